@@ -267,48 +267,210 @@ __global__ void k_precond(const double* __restrict__ g, double* __restrict__ pre
 // ---------------------------------------------------------------------------
 // Tall-skinny products for Gram-Schmidt and the subspace matrix:
 //   part[b][i][j] = sum_{p in chunk b} A[i][p] * B[j][p], i < m, j < n
-// One CTA = one 32 x 32 output tile over a point chunk; fixed summation order.
+// One CTA = one 32 x 32 output tile over a point chunk; its four groups of 64
+// threads take the chunk's 16-point slabs in turn (4 x 4 outputs a thread: 8
+// shared loads per 16 FMA, the LSU and FP64 pipes even) and are added in group
+// order.  Bound by reading A and B; the chunks are cut so that about four CTAs
+// per SM run (24 orbitals of 48^3: 7 CTAs of 16384 points took 649 us a product).
+// upper: tiles below the diagonal are left out (their part is not written).
 // ---------------------------------------------------------------------------
-constexpr int GT = 32, GK = 64;
+constexpr int GT = 32, GK = 16;
 __global__ void __launch_bounds__(256) k_gram_part(const double* __restrict__ A, int m, const double* __restrict__ B,
-                                                   int n, long npts, long chunk, double* __restrict__ part) {
-  __shared__ double As[GT][GK + 1], Bs[GT][GK + 1];
+                                                   int n, long npts, long chunk, int upper,
+                                                   double* __restrict__ part) {
   const int ti = blockIdx.x, tj = blockIdx.y, b = blockIdx.z;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // each thread: 2 x 2 outputs
+  if (upper && ti > tj) return;
+  __shared__ double S[2][4][GT][GK + 1];  // slabs of A and B per group; the sums reuse them
+  const int g = threadIdx.x >> 6, u = threadIdx.x & 63, tx = u & 7, ty = u >> 3;
+  const int kl = u & (GK - 1), rl = u / GK;
   const long p0 = (long)b * chunk, p1 = min(npts, p0 + chunk);
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-  for (long pp = p0; pp < p1; pp += GK) {
-    for (int c = threadIdx.x; c < GT * GK; c += 256) {
-      const int r = c / GK, k = c % GK;
+  double acc[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+  for (long pp = p0 + g * GK; pp < p0 + chunk; pp += 4 * GK) {
+    const long p = pp + kl;
+#pragma unroll
+    for (int r = rl; r < GT; r += 64 / GK) {
       const int i = ti * GT + r, j = tj * GT + r;
-      const long p = pp + k;
-      As[r][k] = (i < m && p < p1) ? A[(long)i * npts + p] : 0.0;
-      Bs[r][k] = (j < n && p < p1) ? B[(long)j * npts + p] : 0.0;
+      S[0][g][r][kl] = (i < m && p < p1) ? A[(long)i * npts + p] : 0.0;
+      S[1][g][r][kl] = (j < n && p < p1) ? B[(long)j * npts + p] : 0.0;
     }
     __syncthreads();
-#pragma unroll 8
+#pragma unroll 4
     for (int k = 0; k < GK; ++k) {
-      const double a0 = As[2 * ty][k], a1 = As[2 * ty + 1][k];
-      const double b0 = Bs[2 * tx][k], b1 = Bs[2 * tx + 1][k];
-      acc[0][0] += a0 * b0;
-      acc[0][1] += a0 * b1;
-      acc[1][0] += a1 * b0;
-      acc[1][1] += a1 * b1;
+      double x[4], y[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        x[r] = S[0][g][ty + 8 * r][k];
+        y[r] = S[1][g][tx + 8 * r][k];
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = fma(x[r], y[c], acc[r][c]);
     }
     __syncthreads();
   }
-  for (int u = 0; u < 2; ++u)
-    for (int v = 0; v < 2; ++v) {
-      const int i = ti * GT + 2 * ty + u, j = tj * GT + 2 * tx + v;
-      if (i < m && j < n) part[((long)b * m + i) * n + j] = acc[u][v];
-    }
+  double* sum = &S[0][0][0][0];  // [4][32 x 32] of the 2 x 4 x 32 x 17 doubles
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sum[g * GT * GT + (ty + 8 * r) * GT + tx + 8 * c] = acc[r][c];
+  __syncthreads();
+  for (int q = threadIdx.x; q < GT * GT; q += 256) {
+    const int i = ti * GT + q / GT, j = tj * GT + q % GT;
+    if (i < m && j < n)
+      part[((long)b * m + i) * n + j] = ((sum[q] + sum[GT * GT + q]) + sum[2 * GT * GT + q]) + sum[3 * GT * GT + q];
+  }
 }
 
-__global__ void k_gram_final(const double* __restrict__ part, int nb, long mn, double scale, double* __restrict__ out) {
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < mn; q += (long)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += part[(long)b * mn + q];
-    out[q] = s * scale;
+// out[q] = scale * sum_b part[b][q]: 32 entries x 32 slices of the chunks per
+// block, the slices added in order
+__global__ void __launch_bounds__(1024) k_gram_final(const double* __restrict__ part, int nb, long mn, double scale,
+                                                     double* __restrict__ out) {
+  __shared__ double red[32][33];
+  const long q = blockIdx.x * 32L + threadIdx.x;
+  double s = 0.0;
+  if (q < mn)
+    for (int b = threadIdx.y; b < nb; b += 32) s += part[(long)b * mn + q];
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && q < mn) {
+    double t = 0.0;
+    for (int k = 0; k < 32; ++k) t += red[k][threadIdx.x];
+    out[q] = t * scale;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Column Gram-Schmidt of all orbitals at once: with G = X^T X hvol the
+// coefficients of every column follow from G alone.  k_gs_coeff (one CTA)
+// eliminates row after row: row i < j of column j holds T(i, j), the part of
+// the original orbital i in the orthonormal orbital j, rows i >= j what is left
+// of G, so one n x n matrix W (row-major) carries both.  The coefficients
+// carry the rounding of G times the growth |T_ij| |x_i|; when that passes
+// GS_GROWTH (orbitals close to linear dependence, or a zero or non-finite one)
+// *bad is set and the caller takes the column-by-column form instead.  24
+// orbitals of 48^3: 115 launches, 15.7 ms column by column; 5 launches here
+// (a solver iteration with CG and subspace rotation 18.8 -> 2.1 ms).
+// ---------------------------------------------------------------------------
+constexpr double GS_GROWTH = 100.0;  // largest |T_ij| |x_i|: two digits of the 16
+constexpr int GC_THREADS = 512;
+constexpr int GC_SMEM_N = 150;  // W kept in shared memory up to here (180 KB)
+
+__global__ void __launch_bounds__(GC_THREADS) k_gs_coeff(double* __restrict__ G, int n, int in_smem,
+                                                         double* __restrict__ T, double* __restrict__ work,
+                                                         int* __restrict__ bad) {
+  extern __shared__ double gsm[];
+  double* nrm = work;        // [n] G_ii
+  double* rb = work + n;     // [n] R(j, k) of the current row
+  double* W = G;
+  if (in_smem) {
+    W = gsm;
+    nrm = gsm + (size_t)n * n;
+    rb = nrm + n;
+    for (int q = threadIdx.x; q < n * n; q += GC_THREADS) W[q] = G[q];
+  }
+  __shared__ int sbad;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, NWP = GC_THREADS / 32;
+  if (threadIdx.x == 0) sbad = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += GC_THREADS) nrm[i] = W[(size_t)i * n + i];
+  __syncthreads();
+  for (int j = 0; j < n; ++j) {
+    const double d = W[(size_t)j * n + j];
+    const double r = 1.0 / sqrt(d);  // a negative or NaN d is caught by the growth test
+    for (int k = j + 1 + threadIdx.x; k < n; k += GC_THREADS) rb[k] = W[(size_t)j * n + k] * r;
+    __syncthreads();
+    // row j turns from what is left of G into T; column j of T is scaled
+    for (int i = threadIdx.x; i <= j; i += GC_THREADS) W[(size_t)i * n + j] = (i == j) ? r : W[(size_t)i * n + j] * r;
+    for (int k = j + 1 + threadIdx.x; k < n; k += GC_THREADS) W[(size_t)j * n + k] = 0.0;
+    __syncthreads();
+    // T(:, k) -= R(j, k) T(:, j) for rows i <= j; G(i, k) -= R(j, i) R(j, k) for j < i <= k
+    for (int i = warp; i < n; i += NWP) {
+      const double f = i <= j ? W[(size_t)i * n + j] : rb[i];
+      for (int k = max(i, j + 1) + lane; k < n; k += 32) W[(size_t)i * n + k] = fma(-f, rb[k], W[(size_t)i * n + k]);
+    }
+    __syncthreads();
+  }
+  int b = 0;
+  for (int i = warp; i < n; i += NWP)
+    for (int j = lane; j < n; j += 32) {
+      const double v = j >= i ? W[(size_t)i * n + j] : 0.0;
+      T[(size_t)j * n + i] = v;  // column-major for k_gs_apply
+      if (!(v * v * nrm[i] <= GS_GROWTH * GS_GROWTH)) b = 1;
+    }
+  if (b) sbad = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) *bad = sbad;
+}
+
+// Sum of 32 values over the 32 lanes of a warp by reduce-scatter: lane L gets
+// the total of value L (31 shuffles, fixed order).
+__device__ __forceinline__ double warp_scatter32(double (&v)[32], int lane) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const bool upper = (lane & off) != 0;
+#pragma unroll
+    for (int i = 0; i < off; ++i) {
+      const double keep = upper ? v[off + i] : v[i];
+      const double send = upper ? v[i] : v[off + i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  return v[0];
+}
+
+// X(p, j) <- sum_{i <= j} X(p, i) T(i, j) in place (a thread owns its point;
+// column tiles from the last to the first), and the sums of squares of every
+// new column over the block's points in part[j][block].  Each X value is read
+// once per column tile and feeds 32 FMA against T broadcast from shared memory.
+constexpr int GA_THREADS = 128;
+__global__ void __launch_bounds__(GA_THREADS) k_gs_apply(double* __restrict__ X, int n, const double* __restrict__ T,
+                                                         long npts, double* __restrict__ part,
+                                                         const int* __restrict__ bad) {
+  if (*bad) return;
+  __shared__ __align__(16) double Ts[GT][GT];
+  __shared__ double red[GA_THREADS / 32][GT];
+  const long p = blockIdx.x * (long)GA_THREADS + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j0 = (n - 1) / GT * GT; j0 >= 0; j0 -= GT) {
+    double acc[GT];
+#pragma unroll
+    for (int u = 0; u < GT; ++u) acc[u] = 0.0;
+    const int iend = min(n, j0 + GT);
+    for (int i0 = 0; i0 < iend; i0 += GT) {
+      __syncthreads();
+      for (int c = threadIdx.x; c < GT * GT; c += GA_THREADS) {
+        const int ii = c % GT, jj = c / GT;
+        Ts[ii][jj] = (i0 + ii < n && j0 + jj < n) ? T[(size_t)(j0 + jj) * n + i0 + ii] : 0.0;
+      }
+      __syncthreads();
+      if (p < npts) {
+        const int im = min(GT, n - i0);
+#pragma unroll 4
+        for (int ii = 0; ii < im; ++ii) {
+          const double x = X[(long)(i0 + ii) * npts + p];
+#pragma unroll
+          for (int u = 0; u < GT; ++u) acc[u] = fma(x, Ts[ii][u], acc[u]);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < GT; ++u) {
+      if (p < npts && j0 + u < n) X[(long)(j0 + u) * npts + p] = acc[u];
+      acc[u] *= acc[u];
+    }
+    const double s = warp_scatter32(acc, lane);
+    red[warp][lane] = s;
+    __syncthreads();
+    if (threadIdx.x < GT && j0 + threadIdx.x < n) {
+      double t = red[0][threadIdx.x];
+      for (int w = 1; w < GA_THREADS / 32; ++w) t += red[w][threadIdx.x];
+      part[(long)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
+    }
   }
 }
 
@@ -350,15 +512,17 @@ __global__ void k_axpy(double* __restrict__ y, const double* __restrict__ x, dou
     y[i] = a * x[i] + y[i];
 }
 
-// single vector: partial sums of squares, then scale by 1/sqrt(hvol * sum)
+// partial sums of squares of columns blockIdx.y of y, then every column scaled by
+// 1/sqrt(hvol * sum): all columns in one launch each
 __global__ void __launch_bounds__(RT) k_sq_part(const double* __restrict__ y, long n, double* __restrict__ part) {
   __shared__ double red[RT];
   double s = 0.0;
   const long p0 = (long)blockIdx.x * DOT_PTS;
+  const double* yc = y + blockIdx.y * n;
   for (int it = 0; it < DOT_PTS / RT; ++it) {
     const long p = p0 + it * RT + threadIdx.x;
     if (p >= n) break;
-    s += y[p] * y[p];
+    s += yc[p] * yc[p];
   }
   red[threadIdx.x] = s;
   __syncthreads();
@@ -366,19 +530,30 @@ __global__ void __launch_bounds__(RT) k_sq_part(const double* __restrict__ y, lo
     if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+  if (threadIdx.x == 0) part[(long)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
 }
 
-__global__ void k_scale_norm(double* __restrict__ y, long n, const double* __restrict__ part, int nblk, double hvol) {
-  __shared__ double f;
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += part[b];
-    f = 1.0 / sqrt(s * hvol);
-  }
+// bad: null, or a device flag that makes the launch return at once
+__global__ void __launch_bounds__(RT) k_scale_norm(const double* y, double* out, long n,
+                                                   const double* __restrict__ part, int nblk, double hvol,
+                                                   const int* __restrict__ bad) {
+  if (bad && *bad) return;
+  __shared__ double red[RT];
+  const double* pc = part + (long)blockIdx.y * nblk;
+  double s = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += RT) s += pc[b];
+  red[threadIdx.x] = s;
   __syncthreads();
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    y[i] = f * y[i];
+  for (int st = RT / 2; st > 0; st >>= 1) {
+    if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
+    __syncthreads();
+  }
+  const double f = 1.0 / sqrt(red[0] * hvol);
+  const long p0 = (long)blockIdx.x * DOT_PTS, base = blockIdx.y * n;
+  for (int it = 0; it < DOT_PTS / RT; ++it) {
+    const long p = p0 + it * RT + threadIdx.x;
+    if (p < n) out[base + p] = f * y[base + p];
+  }
 }
 
 __global__ void k_relayout_real(const double* __restrict__ src, double* __restrict__ dst, int nx, int ny, int nz,
@@ -531,7 +706,6 @@ int gs_precond(sb200_ctx* c, const double* g, double* pre, double alpha) {
   return SB200_OK;
 }
 
-// C (m x n, row-major [i][j]) = scale * A(m orbitals) . B(n orbitals)
 // ---- complex column Gram-Schmidt (gram_schmidt_col_complex8) -------------
 // Orbitals io of one (k, spin) group sit `stride` complex values apart.
 // part[io2][b] = sum over the points of block b of conj(psi_io2) psi_io1
@@ -619,22 +793,30 @@ __global__ void k_zscale_norm(double2* __restrict__ y, long n, const double* __r
     y[p] = make_double2(sc * y[p].x, sc * y[p].y);
 }
 
-int gs_gram(sb200_ctx* c, const double* A, int m, const double* B, int n, double scale, double* C_dev) {
+// C (m x n, row-major [i][j]) = scale * A(m orbitals) . B(n orbitals); upper:
+// entries of 32 x 32 tiles below the diagonal are left undefined
+int gs_gram(sb200_ctx* c, const double* A, int m, const double* B, int n, double scale, double* C_dev,
+            bool upper = false) {
   const long npts = c->g.npts;
-  int nb = (int)((npts + 16383) / 16384);
-  if (nb > 64) nb = 64;
-  const long chunk = ((npts + nb - 1) / nb + GK - 1) / GK * GK;
-  nb = (int)((npts + chunk - 1) / chunk);
+  const long ti = (m + GT - 1) / GT, tj = (n + GT - 1) / GT;
+  // about four CTAs per SM, each with at least 256 points
+  long nb = (148L * 4 + ti * tj - 1) / (ti * tj);
+  if (nb > (npts + 255) / 256) nb = (npts + 255) / 256;
+  if (nb < 1) nb = 1;
+  const long chunk = ((npts + nb - 1) / nb + 4 * GK - 1) / (4 * GK) * (4 * GK);
+  nb = (npts + chunk - 1) / chunk;
   const size_t need = (size_t)nb * m * n;
   if (c->gs.gram_cap < need) {
     dfree(c->gs.d_gram);
+    c->gs.gram_cap = 0;
     TRY_GS(dalloc(&c->gs.d_gram, need));
     c->gs.gram_cap = need;
   }
-  dim3 g((m + GT - 1) / GT, (n + GT - 1) / GT, nb);
-  k_gram_part<<<g, 256, 0, c->stream>>>(A, m, B, n, npts, chunk, c->gs.d_gram);
+  dim3 g((unsigned)ti, (unsigned)tj, (unsigned)nb);
+  k_gram_part<<<g, 256, 0, c->stream>>>(A, m, B, n, npts, chunk, upper ? 1 : 0, c->gs.d_gram);
   SB_LAUNCH_CHECK("k_gram_part");
-  k_gram_final<<<gridsz((long)m * n), 256, 0, c->stream>>>(c->gs.d_gram, nb, (long)m * n, scale, C_dev);
+  const long mn = (long)m * n;
+  k_gram_final<<<(unsigned)((mn + 31) / 32), dim3(32, 32), 0, c->stream>>>(c->gs.d_gram, (int)nb, mn, scale, C_dev);
   SB_LAUNCH_CHECK("k_gram_final");
   return SB200_OK;
 }
@@ -688,13 +870,45 @@ int gs_rotate_sub(sb200_ctx* c, const double* X, int m, const double* coeff_dev,
   return SB200_OK;
 }
 
-// y <- y / sqrt(hvol * sum y^2), one orbital, deterministic
-int gs_norm_scale(sb200_ctx* c, double* y) {
+// out_j <- y_j / sqrt(hvol * sum y_j^2) for nc orbitals, deterministic
+int gs_norm_scale(sb200_ctx* c, const double* y, double* out, int nc) {
   const long n = c->g.npts;
   const int nblk = (int)((n + DOT_PTS - 1) / DOT_PTS);
-  k_sq_part<<<nblk, RT, 0, c->stream>>>(y, n, c->gs.d_part);
+  dim3 g(nblk, nc);
+  k_sq_part<<<g, RT, 0, c->stream>>>(y, n, c->gs.d_part);
   SB_LAUNCH_CHECK("k_sq_part");
-  k_scale_norm<<<gridsz(n), 256, 0, c->stream>>>(y, n, c->gs.d_part, nblk, c->g.hvol);
+  k_scale_norm<<<g, RT, 0, c->stream>>>(y, out, n, c->gs.d_part, nblk, c->g.hvol, nullptr);
+  SB_LAUNCH_CHECK("k_scale_norm");
+  return SB200_OK;
+}
+
+// Gram-Schmidt of the n contiguous orbitals X at once (k_gs_coeff); *bad (device)
+// says that X was left as it was and needs the column form.  mat: 2 n^2 + 2 n
+// doubles.
+int gs_orthonormalise(sb200_ctx* c, double* X, int n, double* mat, int* bad) {
+  const long npts = c->g.npts;
+  double* G = mat;
+  double* T = mat + (size_t)n * n;
+  double* work = T + (size_t)n * n;
+  TRY_GS(gs_gram(c, X, n, X, n, c->g.hvol, G, true));
+  const int in_smem = n <= GC_SMEM_N;
+  const size_t smem = in_smem ? ((size_t)n * n + 2 * n) * sizeof(double) : 0;
+  SB_CUDA(cudaFuncSetAttribute(k_gs_coeff, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (GC_SMEM_N * GC_SMEM_N + 2 * GC_SMEM_N) * (int)sizeof(double)));
+  k_gs_coeff<<<1, GC_THREADS, smem, c->stream>>>(G, n, in_smem, T, work, bad);
+  SB_LAUNCH_CHECK("k_gs_coeff");
+  const int nblk = (int)((npts + GA_THREADS - 1) / GA_THREADS);
+  const size_t need = (size_t)nblk * n;  // the sums of squares share the Gram partials' buffer
+  if (c->gs.gram_cap < need) {
+    dfree(c->gs.d_gram);
+    c->gs.gram_cap = 0;
+    TRY_GS(dalloc(&c->gs.d_gram, need));
+    c->gs.gram_cap = need;
+  }
+  k_gs_apply<<<nblk, GA_THREADS, 0, c->stream>>>(X, n, T, npts, c->gs.d_gram, bad);
+  SB_LAUNCH_CHECK("k_gs_apply");
+  k_scale_norm<<<dim3((unsigned)((npts + DOT_PTS - 1) / DOT_PTS), n), RT, 0, c->stream>>>(X, X, npts, c->gs.d_gram,
+                                                                                       nblk, c->g.hvol, bad);
   SB_LAUNCH_CHECK("k_scale_norm");
   return SB200_OK;
 }
@@ -858,8 +1072,10 @@ int sb200_gram_schmidt_real(sb200_ctx* c, double* psi) {
   TRY_GS(gs_ensure(c, false));
   const int nspin = c->orb.nspin, no = c->orb.no;
   const long npts = c->g.npts;
-  TRY_GS(gs_mat(c, (size_t)no + 8));
+  const size_t nn = (size_t)no * no;
+  TRY_GS(gs_mat(c, 2 * nn + 2 * (size_t)no + 8));
   double* coeff = c->gs.d_mat;
+  int* bad = (int*)(c->gs.d_mat + 2 * nn + 2 * (size_t)no);
   // orbitals of one spin are strided by nspin blocks: gather per spin
   double* buf = nullptr;
   if (nspin > 1) {
@@ -874,14 +1090,18 @@ int sb200_gram_schmidt_real(sb200_ctx* c, double* psi) {
                                 cudaMemcpyDeviceToDevice, c->stream));
       P = buf;
     }
-    for (int io1 = 0; io1 < no; ++io1) {
+    TRY_GS(gs_orthonormalise(c, P, no, c->gs.d_mat, bad));
+    int hbad = 0;
+    SB_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    SB_CUDA(cudaStreamSynchronize(c->stream));
+    for (int io1 = 0; hbad && io1 < no; ++io1) {  // close to linear dependence: column by column
       double* w1 = P + npts * io1;
       if (io1 > 0) {
         // coeff(io2) = hvol <psi_io2 | psi_io1>, io2 < io1 ; w1 -= sum coeff * psi_io2
         TRY_GS(gs_gram(c, P, io1, w1, 1, c->g.hvol, coeff));
         TRY_GS(gs_rotate_sub(c, P, io1, coeff, w1));
       }
-      TRY_GS(gs_norm_scale(c, w1));
+      TRY_GS(gs_norm_scale(c, w1, w1, 1));
     }
     if (nspin > 1)
       for (int io = 0; io < no; ++io)
@@ -966,7 +1186,6 @@ int sb200_subspace_diag_real(sb200_ctx* c, double* psi, double* evals) {
   DevGuard dg(c->device);
   TRY_GS(gs_ensure(c, true));
   const int nspin = c->orb.nspin, no = c->orb.no;
-  const long npts = c->g.npts;
   if (nspin != 1) return set_error(SB200_ERR_UNSUPPORTED, "subspace diagonalisation implemented for nspin = 1");
   double* hpsi = c->gs.d_work;
   double* rot = c->gs.d_work + c->gs.n;
@@ -979,13 +1198,12 @@ int sb200_subspace_diag_real(sb200_ctx* c, double* psi, double* evals) {
   double* ework = M + 2 * nn;
   double* w = M + 4 * nn;
   int* info = (int*)(w + no);
-  TRY_GS(gs_gram(c, psi, no, hpsi, no, c->g.hvol, M));
+  TRY_GS(gs_gram(c, psi, no, hpsi, no, c->g.hvol, M, true));
   // M[i][j] row-major = <psi_i|H psi_j>; the eigensolver reads its upper
   // triangle (dsyev with uplo = 'U'), on the GPU
   TRY_GS(launch_eigh(c, M, no, ework, V, w, info));
   TRY_GS(gs_rotate(c, psi, no, V, no, 0.0, rot));
-  for (int io = 0; io < no; ++io) TRY_GS(gs_norm_scale(c, rot + npts * io));
-  SB_CUDA(cudaMemcpyAsync(psi, rot, sizeof(double) * npts * no, cudaMemcpyDeviceToDevice, c->stream));
+  TRY_GS(gs_norm_scale(c, rot, psi, no));
   std::vector<double> hw(no + 1);
   SB_CUDA(cudaMemcpyAsync(hw.data(), w, sizeof(double) * (no + 1), cudaMemcpyDeviceToHost, c->stream));
   SB_CUDA(cudaStreamSynchronize(c->stream));

@@ -131,3 +131,28 @@ def test_subspace_diag_gpu_eigensolver(no):
     np.testing.assert_allclose(Y.T @ Y * s.grid.hvol, np.eye(no), atol=1e-11)
     D = Y.T @ HY * s.grid.hvol
     assert np.max(np.abs(D - np.diag(w_ref))) <= 1e-9 * max(1.0, np.max(np.abs(w_ref)))
+
+
+@pytest.mark.parametrize("no,dependence", [(1, 0.0), (31, 0.0), (32, 0.0), (33, 0.0), (65, 0.0), (151, 0.0), (20, 1e-3)],
+                         ids=lambda v: str(v))
+def test_gram_schmidt_real_all_columns_at_once(no, dependence):
+    """Gram-Schmidt of all columns from one Gram matrix, at the edges of its
+    32-column tiles and past the coefficients' shared-memory size, and (last
+    case) orbitals so close to dependent that the column-by-column form takes
+    over.  Tolerance: both forms keep rounding times the growth |T_ij| |x_i|,
+    at most 100 in the one and 1 / dependence in the other, over `no` terms."""
+    s = synth.isolated_system(num=(18, 17, 19), no=no, natom=1, seed=60 + no, real=True, name=f"gsall{no}")
+    rng = np.random.default_rng(7)
+    psi0 = s.psi + 0.2 * rng.standard_normal(s.psi.shape) * (s.psi != 0)
+    if dependence:
+        psi0[..., 5, 0] = psi0[..., 2, 0] + dependence * psi0[..., 5, 0]
+    ref = Oracle(s).gram_schmidt_real(psi0)
+    ctx = _ctx(s)
+    psi = ctx.gs_upload(psi0)
+    ctx.gram_schmidt_real(psi)
+    out = ctx.gs_download(psi)
+    growth = 1.0 / dependence if dependence else 100.0
+    assert S.rel_err(out, ref) < 4 * no * growth * 2.2e-16
+    sl = s.grid.interior_slices()
+    X = np.stack([out[sl + (0, i, 0)].ravel() for i in range(no)], axis=1)
+    np.testing.assert_allclose(X.T @ X * s.grid.hvol, np.eye(no), atol=4 * no * growth * 2.2e-16)
