@@ -27,8 +27,11 @@
 namespace sb200 {
 namespace {
 
-constexpr int ET = 512;  // threads of the eigensolver CTA
+constexpr int ET = 512;         // threads of the eigensolver CTA
+constexpr int ET_SMALL = 128;   // for n <= ESM_N: the barriers of its many short steps cost less
+constexpr int ESM_N = 64;       // A and Z in shared memory up to here (64 KB)
 
+template <int ET>
 __device__ __forceinline__ double block_sum(double v, double* red) {
   // fixed-order tree over the CTA (warp butterfly, then warps in order)
 #pragma unroll
@@ -45,10 +48,15 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // M: n x n, row-major <psi_i|H psi_j> (its upper triangle is used, as dsyev
 // with uplo = 'U').  A: n x n work (column-major).  V: eigenvectors, V[i n + k]
 // = component k of eigenvector i.  w: eigenvalues.  sm: 5 n doubles.
-__global__ void __launch_bounds__(ET, 1) k_eigh(const double* __restrict__ M, int n, double* __restrict__ A,
-                                                double* __restrict__ Z, double* __restrict__ V,
-                                                double* __restrict__ w, int* __restrict__ info) {
+template <int ET, bool SMEM>
+__global__ void __launch_bounds__(ET, 1) k_eigh(const double* __restrict__ M, int n, double* A, double* Z,
+                                                double* __restrict__ V, double* __restrict__ w,
+                                                int* __restrict__ info) {
   extern __shared__ double sm[];
+  if (SMEM) {
+    A = sm + 5 * n;
+    Z = A + n * n;
+  }
   double* d = sm;          // [n] diagonal
   double* e = d + n;       // [n] subdiagonal e[i] = T(i+1, i), e[n-1] = 0
   double* tau = e + n;     // [n] reflection factors
@@ -71,7 +79,7 @@ __global__ void __launch_bounds__(ET, 1) k_eigh(const double* __restrict__ M, in
     const int m = n - k - 1;  // length of the column below the diagonal
     double s2 = 0.0;
     for (int i = 1 + t; i < m; i += ET) s2 += a(k + 1 + i, k) * a(k + 1 + i, k);
-    const double tail = block_sum(s2, red);
+    const double tail = block_sum<ET>(s2, red);
     const double x0 = a(k + 1, k);
     if (tail == 0.0) {  // already tridiagonal in this column
       if (t == 0) {
@@ -101,7 +109,7 @@ __global__ void __launch_bounds__(ET, 1) k_eigh(const double* __restrict__ M, in
     __syncthreads();
     double vp = 0.0;
     for (int i = t; i < m; i += ET) vp += a(k + 1 + i, k) * a(k, k + 1 + i);
-    const double K = 0.5 * tk * block_sum(vp, red);
+    const double K = 0.5 * tk * block_sum<ET>(vp, red);
     for (int i = t; i < m; i += ET) a(k, k + 1 + i) -= K * a(k + 1 + i, k);  // w
     __syncthreads();
     for (long q = t; q < (long)m * m; q += ET) {
@@ -174,10 +182,20 @@ __global__ void __launch_bounds__(ET, 1) k_eigh(const double* __restrict__ M, in
               s2 = s;
               g = c * e[i];
               h = c * p;
-              r = hypot(p, e[i]);
-              e[i + 1] = s * r;
-              s = e[i] / r;
-              c = p / r;
+              // r = |(p, e)| and (c, s) = (p, e) / r: one reciprocal square root
+              // where the squares neither overflow nor lose bits
+              const double ei = e[i], q = fma(p, p, ei * ei);
+              if (q > 1e-250 && q < 1e250) {
+                const double ir = rsqrt(q);
+                e[i + 1] = s * (q * ir);
+                s = ei * ir;
+                c = p * ir;
+              } else {
+                r = hypot(p, ei);
+                e[i + 1] = s * r;
+                s = ei / r;
+                c = p / r;
+              }
               p = c * d[i] - s * g;
               d[i + 1] = h + s * (c * g + s * d[i]);
               rc[i] = c;
@@ -239,12 +257,15 @@ int launch_eigh(sb200_ctx* c, const double* M, int n, double* work, double* V, d
   if (n < 1) return set_error(SB200_ERR_INVALID_ARG, "eigensolver: n < 1");
   const size_t smem = 5 * (size_t)n * sizeof(double);
   if (smem > 200 * 1024) return set_error(SB200_ERR_UNSUPPORTED, "eigensolver: matrix larger than 5120 x 5120");
-  static bool attr = false;
-  if (!attr) {
-    SB_CUDA(cudaFuncSetAttribute(k_eigh, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
+  if (n <= ESM_N) {
+    const size_t all = smem + 2 * (size_t)n * n * sizeof(double);
+    SB_CUDA(cudaFuncSetAttribute(k_eigh<ET_SMALL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024));
+    k_eigh<ET_SMALL, true><<<1, ET_SMALL, all, c->stream>>>(M, n, nullptr, nullptr, V, w, info);
+    SB_LAUNCH_CHECK("k_eigh");
+    return SB200_OK;
   }
-  k_eigh<<<1, ET, smem, c->stream>>>(M, n, work, work + (size_t)n * n, V, w, info);
+  SB_CUDA(cudaFuncSetAttribute(k_eigh<ET, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  k_eigh<ET, false><<<1, ET, smem, c->stream>>>(M, n, work, work + (size_t)n * n, V, w, info);
   SB_LAUNCH_CHECK("k_eigh");
   return SB200_OK;
 }

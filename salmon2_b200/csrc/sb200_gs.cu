@@ -23,16 +23,19 @@ constexpr int DOT_PTS = RT * 8;    // points per reduction CTA
 
 // ---------------------------------------------------------------------------
 // real hpsi: 25-point Laplacian + V_local (stencil.f90:30-80) and the KB term
-// (nonlocal_potential.f90:26-171), one thread per point, x/y/z neighbours
-// through L1 (tables from the complex path: pmap entries carry uV).
+// (nonlocal_potential.f90:26-171; tables from the complex path: pmap entries
+// carry uV)
 // ---------------------------------------------------------------------------
 struct RArgs {
-  int nx, ny, nz, periodic, nspin, nlma, natom, nps, totpts;
+  int nx, ny, nz, periodic, nspin, nlma, natom, nps, totpts, hz;
   long npts;
   double lap0, lapt[12];
   const double* vloc;
   const int *pmap, *ent_lma;
   const double* ent_uv;
+  int pairs;           // 1: the (point, atom) pair form applies
+  const int *pmap2, *pair_lma;
+  const double* pair_uv;
   const double* proj;  // [norb][nlma]
   const int *atom_start, *mps, *lma_start, *nproj, *pt_lin;
   const double *uv, *rinv;
@@ -48,199 +51,373 @@ __device__ __forceinline__ int wrap(int q, int n, int periodic, bool& ok) {
   return q;
 }
 
-__global__ void __launch_bounds__(256) k_dhpsi(const double* __restrict__ in, double* __restrict__ out, RArgs a) {
-  const long p = blockIdx.x * 256L + threadIdx.x;
-  if (p >= a.npts) return;
-  const int o = blockIdx.y;
-  const int x = (int)(p % a.nx), y = (int)((p / a.nx) % a.ny), z = (int)(p / ((long)a.nx * a.ny));
-  const double* src = in + (long)o * a.npts;
-  const long sy = a.nx, sz = (long)a.nx * a.ny;
-  double v[3];
-  const int c3[3] = {x, y, z}, n3[3] = {a.nx, a.ny, a.nz};
-  const long st3[3] = {1, sy, sz};
+// Block-wide sums of NV values per thread (NT threads); every thread gets the
+// totals (fixed order: butterfly in the warp, then the warps in order).
+template <int NV, int NT>
+__device__ __forceinline__ void block_totals(double (&v)[NV], double (*red)[NT / 32]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double acc = 0.0;
+  for (int i = 0; i < NV; ++i)
 #pragma unroll
-    for (int s = 1; s <= ND; ++s) {
-      bool okp, okm;
-      const int qp = wrap(c3[d] + s, n3[d], a.periodic, okp);
-      const int qm = wrap(c3[d] - s, n3[d], a.periodic, okm);
-      const double tp = okp ? __ldg(src + p + (qp - c3[d]) * st3[d]) : 0.0;
-      const double tm = okm ? __ldg(src + p + (qm - c3[d]) * st3[d]) : 0.0;
-      acc += a.lapt[4 * d + s - 1] * (tp + tm);
-    }
-    v[d] = acc;
+    for (int off = 16; off > 0; off >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], off);
+  __syncthreads();
+  if (lane == 0)
+    for (int i = 0; i < NV; ++i) red[i][warp] = v[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    v[i] = red[i][0];
+    for (int w = 1; w < NT / 32; ++w) v[i] += red[i][w];
   }
-  const double vs = v[2] + (v[1] + v[0]);
-  double h = (__ldg(a.vloc + (long)(o % a.nspin) * a.npts + p) + a.lap0) * __ldg(src + p) - 0.5 * vs;
-  if (a.nlma > 0) {
-    const int pm = __ldg(a.pmap + p);
-    if (pm >= 0) {
-      const double* pj = a.proj + (long)o * a.nlma;
-      const int e1 = (pm >> 8) + (pm & 255);
-      for (int e = pm >> 8; e < e1; ++e) h += pj[__ldg(a.ent_lma + e)] * __ldg(a.ent_uv + e);
-    }
-  }
-  out[(long)o * a.npts + p] = h;
 }
 
-// real projections uVpsi = rinv * sum_j uV(j,ilma) psi(jxyz): warp per (orbital, atom)
+// Sum over the blocks of one orbital's partial sums part[n][NV], by every block
+// that needs it (no launch of its own for a scalar).
+template <int NV>
+__device__ __forceinline__ void part_totals(const double* __restrict__ part, int n, double scale, double (&v)[NV],
+                                            double (*red)[RT / 32]) {
+#pragma unroll
+  for (int i = 0; i < NV; ++i) v[i] = 0.0;
+  for (int b = threadIdx.x; b < n; b += RT)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] += part[(long)b * NV + i];
+  block_totals<NV, RT>(v, red);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) v[i] *= scale;
+}
+
+// Launches of one CTA per 32 x 8 tile x hz planes of an orbital: a thread owns
+// an (x, y) column, no index division per point.
+constexpr int HX = 32, HY = 8;
+__device__ __forceinline__ bool tile_column(int nx, int ny, int& x, int& y) {
+  const int ntx = (nx + HX - 1) / HX;
+  x = (int)(blockIdx.x % ntx) * HX + (int)(threadIdx.x % HX);
+  y = (int)(blockIdx.x / ntx) * HY + (int)(threadIdx.x / HX);
+  return x < nx && y < ny;
+}
+__device__ __forceinline__ long tile_block() { return (long)blockIdx.y * gridDim.x + blockIdx.x; }
+
+// H of real orbitals: each column marches up hz planes with the nine z neighbours
+// in registers, x and y neighbours through L1 (17 loads a point).  The KB term
+// by (point, atom) pairs from projections staged in shared memory, the point
+// map read a plane ahead: a chain of dependent loads per entry (four per pair)
+// held a warp for thousands of cycles at every plane of a sphere.  scale: null, or an
+// orbital's partial sums of <in|in> (nscale blocks): the result is that of
+// in / sqrt(<in|in>).  DOT: partial sums of <x|out> and <in scaled|out> in
+// part[o][block][2].
+constexpr int HMAX_NLMA = 1024;
+template <bool DOT>
+__global__ void __launch_bounds__(HX* HY) k_dhpsi(const double* __restrict__ in, double* __restrict__ out, RArgs a,
+                                                  const double* __restrict__ scale, int nscale, double hvol,
+                                                  const double* __restrict__ xk, double* __restrict__ part) {
+  __shared__ double red[2][RT / 32];
+  __shared__ double sproj[HMAX_NLMA];
+  const int o = blockIdx.z;
+  int x, y;
+  const bool act = tile_column(a.nx, a.ny, x, y);
+  const int z0 = blockIdx.y * a.hz, z1 = min(a.nz, z0 + a.hz);
+  const double* pj = a.proj + (long)o * a.nlma;
+  if (a.nlma > 0 && a.nlma <= HMAX_NLMA) {
+    for (int i = threadIdx.x; i < a.nlma; i += HX * HY) sproj[i] = pj[i];
+    pj = sproj;
+  }
+  double f = 1.0;
+  if (scale) {
+    double t[1];
+    part_totals<1>(scale + (long)o * nscale, nscale, hvol, t, red);
+    f = 1.0 / sqrt(t[0]);
+  }
+  __syncthreads();
+  double d[2] = {0.0, 0.0};
+  if (act) {
+    const double* src = in + (long)o * a.npts;
+    const int plane = a.nx * a.ny, col = x + a.nx * y;
+    int xo[2 * ND], yo[2 * ND];
+    unsigned ok = 0;  // bit per x / y neighbour: inside the grid
+#pragma unroll
+    for (int s = 1; s <= ND; ++s) {
+      bool b0, b1, b2, b3;
+      xo[2 * s - 2] = wrap(x + s, a.nx, a.periodic, b0) - x;
+      xo[2 * s - 1] = wrap(x - s, a.nx, a.periodic, b1) - x;
+      yo[2 * s - 2] = (wrap(y + s, a.ny, a.periodic, b2) - y) * a.nx;
+      yo[2 * s - 1] = (wrap(y - s, a.ny, a.periodic, b3) - y) * a.nx;
+      ok |= ((unsigned)b0 | (unsigned)b1 << 1 | (unsigned)b2 << 2 | (unsigned)b3 << 3) << (4 * (s - 1));
+    }
+    auto ldz = [&](int z) -> double {
+      bool in_grid;
+      const int q = wrap(z, a.nz, a.periodic, in_grid);
+      return in_grid ? __ldg(src + (long)q * plane + col) : 0.0;
+    };
+    const int* map = a.pairs ? a.pmap2 : a.pmap;
+    double w[2 * ND + 1];
+#pragma unroll
+    for (int i = 0; i < 2 * ND; ++i) w[i] = ldz(z0 - ND + i);
+    const double* V = a.vloc + (long)(o % a.nspin) * a.npts;
+    int pn = a.nlma > 0 ? __ldg(map + (long)z0 * plane + col) : -1;
+    for (int z = z0; z < z1; ++z) {
+      w[2 * ND] = ldz(z + ND);
+      const long p = (long)z * plane + col;
+      const double* P = src + p;
+      const int pm = pn;
+      if (a.nlma > 0 && z + 1 < z1) pn = __ldg(map + p + plane);
+      double vx = 0.0, vy = 0.0, vz = 0.0;
+#pragma unroll
+      for (int s = 0; s < ND; ++s) {
+        const double xp = (ok >> (4 * s)) & 1 ? __ldg(P + xo[2 * s]) : 0.0;
+        const double xm = (ok >> (4 * s + 1)) & 1 ? __ldg(P + xo[2 * s + 1]) : 0.0;
+        const double yp = (ok >> (4 * s + 2)) & 1 ? __ldg(P + yo[2 * s]) : 0.0;
+        const double ym = (ok >> (4 * s + 3)) & 1 ? __ldg(P + yo[2 * s + 1]) : 0.0;
+        vx += a.lapt[s] * (xp + xm);
+        vy += a.lapt[ND + s] * (yp + ym);
+        vz += a.lapt[2 * ND + s] * (w[ND + 1 + s] + w[ND - 1 - s]);
+      }
+      const double c = w[ND];
+      double h = (__ldg(V + p) + a.lap0) * c - 0.5 * (vz + (vy + vx));
+      if (pm >= 0) {
+        const int e1 = (pm >> 8) + (pm & 255);
+        if (a.pairs) {
+          for (int e = pm >> 8; e < e1; ++e) {
+            const int lm = __ldg(a.pair_lma + e);
+            const double2 u0 = __ldg((const double2*)a.pair_uv + 2 * e), u1 = __ldg((const double2*)a.pair_uv + 2 * e + 1);
+            const double* q = pj + (lm & 0xffffff);
+            const int np = lm >> 24;
+            h += q[0] * u0.x;
+            if (np > 1) h += q[1] * u0.y;
+            if (np > 2) h += q[2] * u1.x;
+            if (np > 3) h += q[3] * u1.y;
+          }
+        } else {
+          for (int e = pm >> 8; e < e1; ++e) h += pj[__ldg(a.ent_lma + e)] * __ldg(a.ent_uv + e);
+        }
+      }
+      h *= f;
+      out[(long)o * a.npts + p] = h;
+      if (DOT) {
+        d[0] = fma(__ldg(xk + (long)o * a.npts + p), h, d[0]);
+        d[1] = fma(f * c, h, d[1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2 * ND; ++i) w[i] = w[i + 1];
+    }
+  }
+  if (DOT) {
+    block_totals<2, HX * HY>(d, red);
+    if (threadIdx.x < 2)
+      part[((long)o * gridDim.x * gridDim.y + tile_block()) * 2 + threadIdx.x] = d[threadIdx.x];
+  }
+}
+
+// real projections uVpsi = rinv * sum_j uV(j,ilma) psi(jxyz): CTA of four warps
+// per (orbital, atom)
 __global__ void __launch_bounds__(128) k_dproject(const double* __restrict__ in, double* __restrict__ proj, RArgs a) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int atom = blockIdx.x * 4 + warp;
-  if (atom >= a.natom) return;
-  const int o = blockIdx.y;
+  __shared__ double red[4][4];
+  const int atom = blockIdx.x, o = blockIdx.y;
   const double* psi = in + (long)o * a.npts;
   const int start = a.atom_start[atom], m = a.mps[atom];
   const int lma0 = a.lma_start[atom], np = a.nproj[atom];
   for (int q0 = 0; q0 < np; q0 += 4) {
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int j = lane; j < m; j += 32) {
+#pragma unroll 2
+    for (int j = threadIdx.x; j < m; j += 128) {
       const double v = __ldg(psi + a.pt_lin[start + j]);
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (q0 + q < np) acc[q] += __ldg(a.uv + (long)(lma0 + q0 + q) * a.nps + j) * v;
     }
+    block_totals<4, 128>(acc, red);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      for (int off = 16; off > 0; off >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
-    if (lane == 0)
-      for (int q = 0; q < 4; ++q)
-        if (q0 + q < np) proj[(long)o * a.nlma + lma0 + q0 + q] = acc[q] * a.rinv[lma0 + q0 + q];
+      if ((int)threadIdx.x == q && q0 + q < np)
+        proj[(long)o * a.nlma + lma0 + q0 + q] = acc[q] * a.rinv[lma0 + q0 + q];
   }
 }
 
 // ---------------------------------------------------------------------------
-// per-orbital dot products: part[o][b][k] for up to 3 products at once
+// The band-by-band CG (conjugate_gradient.f90) as six launches per iteration,
+// each one pass over the orbitals that forms the scalars it needs from the
+// partial sums the launch before left (per orbital, fixed order) and leaves its
+// own: the scalars cost no launch and no vector is read only for a dot.
+// state [o][CG_NC]: <x|H|x> and <g|g> of the last two iterations.
 // ---------------------------------------------------------------------------
-struct DotArgs {
+struct CgArgs {
   long npts;
-  int nblk, ndot;
-  const double *x0, *y0, *x1, *y1, *x2, *y2;
-  double* part;  // [norb][nblk][3]
+  int nx, ny, nz, periodic, hz;
+  double hvol;
+  double* state;
 };
 
-__global__ void __launch_bounds__(RT) k_dots(DotArgs a) {
-  __shared__ double red[3][RT];
-  const int o = blockIdx.y;
-  const long base = (long)o * a.npts;
-  double s[3] = {0.0, 0.0, 0.0};
-  const long p0 = (long)blockIdx.x * DOT_PTS;
+// g = hx - <x|H|x> x, and its low-pass filter (preconditioning.f90:25-77) when
+// LOWPASS: dir = the (filtered) gradient and partial sums of <dir|g>.  Before
+// that, for iterations past the first, psi = x / sqrt(<x|x>) of the iteration
+// before (when 1e-16 < |<x|x>| <= 1e30).  prev: [nprev][2] sums <x|H|x>, <x|x>.
+template <bool LOWPASS>
+__global__ void __launch_bounds__(HX* HY) k_cg_gradient(CgArgs c, const double* __restrict__ x,
+                                                        const double* __restrict__ hx,
+                                                        const double* __restrict__ prev, int nprev,
+                                                        double* __restrict__ psi, double* __restrict__ dir,
+                                                        double rx2, double ry2, double rz2, double omega_d,
+                                                        double* __restrict__ part) {
+  __shared__ double red[2][RT / 32];
+  const int o = blockIdx.z;
+  int ix, iy;
+  const bool act = tile_column(c.nx, c.ny, ix, iy);
+  const int z0 = blockIdx.y * c.hz, z1 = min(c.nz, z0 + c.hz);
+  double v[2];
+  part_totals<2>(prev + (long)o * nprev * 2, nprev, c.hvol, v, red);
+  const double e = v[0];
+  if (tile_block() == 0 && threadIdx.x == 0) c.state[CG_NC * o + CG_XKHXK] = e;
+  const bool keep = psi && 1e-16 < fabs(v[1]) && fabs(v[1]) <= 1e30;
+  const double root = sqrt(v[1]);
+  double s[1] = {0.0};
+  if (act) {
+    const int plane = c.nx * c.ny;
+    const long col = (long)o * c.npts + ix + (long)c.nx * iy;
+    auto grad = [&](long i, bool ok) -> double { return ok ? __ldg(hx + i) - e * x[i] : 0.0; };
+    bool kxp, kxm, kyp, kym, kz;
+    const int xp = wrap(ix + 1, c.nx, c.periodic, kxp) - ix, xm = wrap(ix - 1, c.nx, c.periodic, kxm) - ix;
+    const int yp = (wrap(iy + 1, c.ny, c.periodic, kyp) - iy) * c.nx, ym = (wrap(iy - 1, c.ny, c.periodic, kym) - iy) * c.nx;
+    int q = wrap(z0 - 1, c.nz, c.periodic, kz);
+    double gm = LOWPASS ? grad(col + (long)q * plane, kz) : 0.0, g = grad(col + (long)z0 * plane, true);
+    for (int z = z0; z < z1; ++z) {
+      const long i = col + (long)z * plane;
+      double gp = 0.0, d = g;
+      if (LOWPASS) {
+        q = wrap(z + 1, c.nz, c.periodic, kz);
+        gp = grad(col + (long)q * plane, kz);
+        const double lap = (grad(i + xp, kxp) - 2.0 * g + grad(i + xm, kxm)) * rx2 +
+                           (grad(i + yp, kyp) - 2.0 * g + grad(i + ym, kym)) * ry2 + (gp - 2.0 * g + gm) * rz2;
+        d = omega_d * (2.0 * g - omega_d * (-0.5 * lap));
+      } else if (z + 1 < z1) {
+        gp = grad(i + plane, true);
+      }
+      if (keep) psi[i] = x[i] / root;
+      dir[i] = d;
+      s[0] = fma(d, g, s[0]);
+      gm = g;
+      g = gp;
+    }
+  }
+  block_totals<1, HX * HY>(s, red);
+  if (threadIdx.x == 0) part[(long)o * gridDim.x * gridDim.y + tile_block()] = s[0];
+}
+
+// partial sums of <u|v>
+__global__ void __launch_bounds__(RT) k_cg_dot(CgArgs c, const double* __restrict__ u, const double* __restrict__ v,
+                                               double* __restrict__ part) {
+  __shared__ double red[1][RT / 32];
+  const long base = (long)blockIdx.y * c.npts;
+  double s[1] = {0.0};
   for (int it = 0; it < DOT_PTS / RT; ++it) {
-    const long p = p0 + it * RT + threadIdx.x;
-    if (p >= a.npts) break;
-    s[0] += a.x0[base + p] * a.y0[base + p];
-    if (a.ndot > 1) s[1] += a.x1[base + p] * a.y1[base + p];
-    if (a.ndot > 2) s[2] += a.x2[base + p] * a.y2[base + p];
+    const long p = (long)blockIdx.x * DOT_PTS + it * RT + threadIdx.x;
+    if (p < c.npts) s[0] = fma(u[base + p], v[base + p], s[0]);
   }
-  for (int k = 0; k < 3; ++k) red[k][threadIdx.x] = s[k];
-  __syncthreads();
-  for (int st = RT / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
-      for (int k = 0; k < 3; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x < 3) a.part[((long)o * a.nblk + blockIdx.x) * 3 + threadIdx.x] = red[threadIdx.x][0];
+  block_totals<1, RT>(s, red);
+  if (threadIdx.x == 0) part[(long)blockIdx.y * gridDim.x + blockIdx.x] = s[0];
 }
 
-__global__ void k_dots_final(const double* __restrict__ part, int norb, int nblk, double hvol, double* __restrict__ out) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= norb) return;
-  for (int k = 0; k < 3; ++k) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += part[((long)o * nblk + b) * 3 + k];
-    out[3 * o + k] = s * hvol;
+// pk = dir + uk pk (uk = 0 where restart) and partial sums of <x|pk>; pgg: the
+// sums of <dir|g>, kept in the state for the next iteration
+__global__ void __launch_bounds__(RT) k_cg_direction(CgArgs c, const double* __restrict__ dir,
+                                                     const double* __restrict__ x, const double* __restrict__ pgg,
+                                                     int ngg, int iter, int restart, double* __restrict__ pk,
+                                                     double* __restrict__ part) {
+  __shared__ double red[1][RT / 32];
+  const int o = blockIdx.y;
+  const long base = (long)o * c.npts;
+  double v[1];
+  part_totals<1>(pgg + (long)o * ngg, ngg, c.hvol, v, red);
+  double uk = 0.0;
+  if (!restart) {
+    const double old = c.state[CG_NC * o + CG_GG0 + ((iter + 1) & 1)];
+    uk = fabs(old) > 1e-16 ? v[0] / old : 0.0;
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) c.state[CG_NC * o + CG_GG0 + (iter & 1)] = v[0];
+  double s[1] = {0.0};
+  for (int it = 0; it < DOT_PTS / RT; ++it) {
+    const long p = (long)blockIdx.x * DOT_PTS + it * RT + threadIdx.x;
+    if (p >= c.npts) break;
+    const double q = restart ? dir[base + p] : dir[base + p] + uk * pk[base + p];
+    pk[base + p] = q;
+    s[0] = fma(x[base + p], q, s[0]);
+  }
+  block_totals<1, RT>(s, red);
+  if (threadIdx.x == 0) part[(long)o * gridDim.x + blockIdx.x] = s[0];
 }
 
-// ---------------------------------------------------------------------------
-// CG vector updates with per-orbital coefficients (conjugate_gradient.f90)
-// ---------------------------------------------------------------------------
-enum { U_GK = 0, U_PK, U_PKO, U_SCALE, U_XH, U_PSI };
-struct UpdArgs {
-  long npts, n;
-  int op;
-  const double* coef;  // per-orbital coefficient block (see k_cg_scalars)
-  double *a, *b, *c, *d;
-};
-
-__global__ void k_cg_update(UpdArgs u) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < u.n; i += (long)gridDim.x * blockDim.x) {
-    const int o = (int)(i / u.npts);
-    const double* cf = u.coef + CG_NC * o;
-    switch (u.op) {
-      case U_GK:  // gk = hxk - xkHxk * xk           (a = gk, b = hxk, c = xk)
-        u.a[i] = u.b[i] - cf[CG_XKHXK] * u.c[i];
-        break;
-      case U_PK:  // pk = g + uk * pk                   (a = pk, b = g or pre_g)
-        u.a[i] = u.b[i] + cf[CG_UK] * u.a[i];
-        break;
-      case U_PKO:  // pko = pk - zs * xk                (a = pko, b = pk, c = xk)
-        u.a[i] = u.b[i] - cf[CG_ZS] * u.c[i];
-        break;
-      case U_SCALE:  // pko = pko / sqrt(sum)
-        u.a[i] = u.a[i] / sqrt(cf[CG_SUM]);
-        break;
-      case U_XH: {  // xk = cx xk + cp pko ; hxk = cx hxk + cp hwf  (a=xk, b=pko, c=hxk, d=hwf)
-        u.a[i] = cf[CG_CX] * u.a[i] + cf[CG_CP] * u.b[i];
-        u.c[i] = cf[CG_CX] * u.c[i] + cf[CG_CP] * u.d[i];
-        break;
-      }
-      case U_PSI: {  // psi = xk / sqrt(xkxk) when 1e-16 < |xkxk| <= 1e30   (a = psi, b = xk)
-        const double q = cf[CG_XKXK];
-        if (1e-16 < fabs(q) && fabs(q) <= 1e30) u.a[i] = u.b[i] / sqrt(q);
-        break;
-      }
-    }
+// pko = pk - <x|pk> x and partial sums of <pko|pko>
+__global__ void __launch_bounds__(RT) k_cg_orthogonal(CgArgs c, const double* __restrict__ pk,
+                                                      const double* __restrict__ x, const double* __restrict__ pxp,
+                                                      double* __restrict__ pko, double* __restrict__ part) {
+  __shared__ double red[1][RT / 32];
+  const int o = blockIdx.y;
+  const long base = (long)o * c.npts;
+  double v[1];
+  part_totals<1>(pxp + (long)o * gridDim.x, gridDim.x, c.hvol, v, red);
+  double s[1] = {0.0};
+  for (int it = 0; it < DOT_PTS / RT; ++it) {
+    const long p = (long)blockIdx.x * DOT_PTS + it * RT + threadIdx.x;
+    if (p >= c.npts) break;
+    const double q = pk[base + p] - v[0] * x[base + p];
+    pko[base + p] = q;
+    s[0] = fma(q, q, s[0]);
   }
+  block_totals<1, RT>(s, red);
+  if (threadIdx.x == 0) part[(long)o * gridDim.x + blockIdx.x] = s[0];
 }
 
-// per-orbital scalar algebra of gscg_rwf; `stage` selects which block of the
-// iteration is being completed; dots = latest k_dots_final output [o][3]
-__global__ void k_cg_scalars(double* __restrict__ coef, const double* __restrict__ dots, int norb, int stage,
-                             int iter) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= norb) return;
-  double* cf = coef + CG_NC * o;
-  const double* d = dots + 3 * o;
-  switch (stage) {
-    case 0:  // initial <xk|H|xk>
-      cf[CG_XKHXK] = d[0];
-      break;
-    case 1: {  // sum = <(pre)g|g>; uk; gkgk = sum
-      const double sum = d[0];
-      cf[CG_UK] = (iter == 1) ? 0.0 : ((fabs(cf[CG_GKGK]) > 1e-16) ? sum / cf[CG_GKGK] : 0.0);
-      cf[CG_GKGK] = sum;
-      break;
-    }
-    case 2:  // zs = <xk|pk>
-      cf[CG_ZS] = d[0];
-      break;
-    case 3:  // sum = <pko|pko>
-      cf[CG_SUM] = d[0];
-      break;
-    case 4: {  // xkHpk, pkHpk -> ev, cx, cp
-      const double xkHxk = cf[CG_XKHXK], xkHpk = d[0], pkHpk = d[1];
-      const double ev = 0.5 * ((xkHxk + pkHpk) - sqrt((xkHxk - pkHpk) * (xkHxk - pkHpk) +
-                                                      4.0 * fabs(xkHpk) * fabs(xkHpk)));
-      double cx, cp;
-      if (fabs(ev - xkHxk) > 1e-16) {
-        cx = xkHpk / (ev - xkHxk);
-        cp = 1.0 / sqrt(1.0 + fabs(cx) * fabs(cx));
-        cx = cx * cp;
-      } else {
-        cx = 1.0;
-        cp = 0.0;
-      }
-      cf[CG_CX] = cx;
-      cf[CG_CP] = cp;
-      break;
-    }
-    case 5:  // xkHxk, xkxk after the update
-      cf[CG_XKHXK] = d[0];
-      cf[CG_XKXK] = d[1];
-      break;
+// 2 x 2 Rayleigh-Ritz of x and pko / sqrt(<pko|pko>): x and hx rotated to the
+// lower state (xin may be psi in the first iteration), partial sums of <x|H|x>, <x|x>
+__global__ void __launch_bounds__(RT) k_cg_rotate(CgArgs c, const double* xin, double* xout,
+                                                  double* __restrict__ hx, const double* __restrict__ pko,
+                                                  const double* __restrict__ hwf, const double* __restrict__ ppp,
+                                                  const double* __restrict__ ph, int nph,
+                                                  double* __restrict__ part) {
+  __shared__ double red[2][RT / 32];
+  const int o = blockIdx.y;
+  const long base = (long)o * c.npts;
+  double n[1], v[2];
+  part_totals<1>(ppp + (long)o * gridDim.x, gridDim.x, c.hvol, n, red);
+  part_totals<2>(ph + (long)o * nph * 2, nph, c.hvol, v, red);
+  const double f = 1.0 / sqrt(n[0]);
+  const double xkHxk = c.state[CG_NC * o + CG_XKHXK], xkHpk = v[0], pkHpk = v[1];
+  const double ev = 0.5 * ((xkHxk + pkHpk) -
+                           sqrt((xkHxk - pkHpk) * (xkHxk - pkHpk) + 4.0 * fabs(xkHpk) * fabs(xkHpk)));
+  double cx = 1.0, cp = 0.0;
+  if (fabs(ev - xkHxk) > 1e-16) {
+    cx = xkHpk / (ev - xkHxk);
+    cp = 1.0 / sqrt(1.0 + fabs(cx) * fabs(cx));
+    cx = cx * cp;
+  }
+  double s[2] = {0.0, 0.0};
+  for (int it = 0; it < DOT_PTS / RT; ++it) {
+    const long p = (long)blockIdx.x * DOT_PTS + it * RT + threadIdx.x;
+    if (p >= c.npts) break;
+    const double xn = cx * xin[base + p] + cp * (f * pko[base + p]);
+    const double hn = cx * hx[base + p] + cp * hwf[base + p];
+    xout[base + p] = xn;
+    hx[base + p] = hn;
+    s[0] = fma(xn, hn, s[0]);
+    s[1] = fma(xn, xn, s[1]);
+  }
+  block_totals<2, RT>(s, red);
+  if (threadIdx.x < 2) part[((long)o * gridDim.x + blockIdx.x) * 2 + threadIdx.x] = s[threadIdx.x];
+}
+
+// psi = x / sqrt(<x|x>) after the last iteration; esp[o] = <x|H|x> / <x|x>
+__global__ void __launch_bounds__(RT) k_cg_end(CgArgs c, const double* __restrict__ x,
+                                               const double* __restrict__ prev, int nprev, double* __restrict__ psi,
+                                               double* __restrict__ esp) {
+  __shared__ double red[2][RT / 32];
+  const int o = blockIdx.y;
+  const long base = (long)o * c.npts;
+  double v[2];
+  part_totals<2>(prev + (long)o * nprev * 2, nprev, c.hvol, v, red);
+  if (blockIdx.x == 0 && threadIdx.x == 0) esp[o] = v[0] / v[1];
+  if (!(1e-16 < fabs(v[1]) && fabs(v[1]) <= 1e30)) return;
+  const double root = sqrt(v[1]);
+  for (int it = 0; it < DOT_PTS / RT; ++it) {
+    const long p = (long)blockIdx.x * DOT_PTS + it * RT + threadIdx.x;
+    if (p < c.npts) psi[base + p] = x[base + p] / root;
   }
 }
 
@@ -506,12 +683,6 @@ __global__ void __launch_bounds__(256) k_rotate(const double* __restrict__ X, in
       }
 }
 
-// y[p] = y[p] - x[p] * coef  (one orbital) and norm handled by dots
-__global__ void k_axpy(double* __restrict__ y, const double* __restrict__ x, double a, long n) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    y[i] = a * x[i] + y[i];
-}
-
 // partial sums of squares of columns blockIdx.y of y, then every column scaled by
 // 1/sqrt(hvol * sum): all columns in one launch each
 __global__ void __launch_bounds__(RT) k_sq_part(const double* __restrict__ y, long n, double* __restrict__ part) {
@@ -586,6 +757,7 @@ static RArgs rargs(sb200_ctx* c) {
   a.ny = c->g.ny;
   a.nz = c->g.nz;
   a.periodic = c->g.periodic;
+  a.hz = 1;
   a.nspin = c->orb.nspin;
   a.nlma = c->pp.nlma;
   a.natom = c->pp.natom;
@@ -598,6 +770,10 @@ static RArgs rargs(sb200_ctx* c) {
   a.pmap = c->pp.d_pmap;
   a.ent_lma = c->pp.d_ent_lma;
   a.ent_uv = c->pp.d_ent_uv;
+  a.pairs = c->pp.npair > 0 ? 1 : 0;
+  a.pmap2 = c->pp.d_pmap2;
+  a.pair_lma = c->pp.d_pair_lma;
+  a.pair_uv = c->pp.d_pair_uv;
   a.proj = c->gs.d_proj;
   a.atom_start = c->pp.d_atom_start;
   a.mps = c->pp.d_mps;
@@ -609,26 +785,48 @@ static RArgs rargs(sb200_ctx* c) {
   return a;
 }
 
+// one CTA per 32 x 8 tile x hz planes and orbital; hz from 1 (small grids: latency)
+// to 16 (a column reads 8 planes more than it has), about six CTAs per SM
+int dhpsi_hz(const sb200_ctx* c) {
+  const GridInfo& g = c->g;
+  const long planes = (long)((g.nx + HX - 1) / HX) * ((g.ny + HY - 1) / HY) * g.nz * c->orb.norb;
+  const long hz = planes / (148 * 6);
+  return (int)(hz < 1 ? 1 : (hz > 16 ? 16 : hz));
+}
+dim3 dhpsi_grid(const sb200_ctx* c) {
+  const GridInfo& g = c->g;
+  const int hz = dhpsi_hz(c);
+  return dim3((unsigned)(((g.nx + HX - 1) / HX) * ((g.ny + HY - 1) / HY)), (unsigned)((g.nz + hz - 1) / hz),
+              (unsigned)c->orb.norb);
+}
+
 int gs_ensure(sb200_ctx* c, bool cg_work) {
   GSState& s = c->gs;
   const long n = c->g.npts * c->orb.norb;
   const int norb = c->orb.norb;
   const int nblk = (int)((c->g.npts + DOT_PTS - 1) / DOT_PTS);
-  if (s.n != n || s.norb != norb) {
+  const dim3 hg = dhpsi_grid(c);
+  const size_t per = 6 * (size_t)nblk + 3 * (size_t)hg.x * hg.y;  // partial sums of an orbital
+  const size_t npart = per * norb, nproj = (size_t)norb * (c->pp.nlma > 0 ? c->pp.nlma : 1);
+  if (s.n != n || s.norb != norb || s.npart < npart || s.nproj < nproj) {
     dfree(s.d_proj);
     dfree(s.d_part);
     dfree(s.d_dots);
     dfree(s.d_coef);
     dfree(s.d_work);
+    s.n = 0;
+    s.have_work = false;
+    TRY_GS(dalloc(&s.d_proj, nproj));
+    TRY_GS(dalloc(&s.d_part, npart));
+    TRY_GS(dalloc(&s.d_dots, (size_t)norb));
+    TRY_GS(dalloc(&s.d_coef, (size_t)norb * CG_NC));
     s.n = n;
     s.norb = norb;
     s.nblk = nblk;
-    s.have_work = false;
-    TRY_GS(dalloc(&s.d_proj, (size_t)norb * (c->pp.nlma > 0 ? c->pp.nlma : 1)));
-    TRY_GS(dalloc(&s.d_part, (size_t)norb * nblk * 3));
-    TRY_GS(dalloc(&s.d_dots, (size_t)norb * 3));
-    TRY_GS(dalloc(&s.d_coef, (size_t)norb * CG_NC));
+    s.npart = npart;
+    s.nproj = nproj;
   }
+  s.nblk = nblk;
   if (cg_work && !s.have_work) {
     TRY_GS(dalloc(&s.d_work, (size_t)n * 7));
     s.have_work = true;
@@ -636,62 +834,23 @@ int gs_ensure(sb200_ctx* c, bool cg_work) {
   return SB200_OK;
 }
 
-int gs_hpsi(sb200_ctx* c, const double* in, double* out) {
+// out = H in; with part: partial sums of <x|out> and <in|out>; with scale
+// (partial sums of <in|in>): of in / sqrt(<in|in>)
+int gs_hpsi(sb200_ctx* c, const double* in, double* out, const double* scale = nullptr, const double* x = nullptr,
+            double* part = nullptr) {
   RArgs a = rargs(c);
+  a.hz = dhpsi_hz(c);
   if (a.nlma > 0) {
-    dim3 g((a.natom + 3) / 4, c->orb.norb);
+    dim3 g(a.natom, c->orb.norb);
     k_dproject<<<g, 128, 0, c->stream>>>(in, c->gs.d_proj, a);
     SB_LAUNCH_CHECK("k_dproject");
   }
-  dim3 g((unsigned)((a.npts + 255) / 256), c->orb.norb);
-  k_dhpsi<<<g, 256, 0, c->stream>>>(in, out, a);
+  const dim3 g = dhpsi_grid(c);
+  if (part)
+    k_dhpsi<true><<<g, HX * HY, 0, c->stream>>>(in, out, a, scale, c->gs.nblk, c->g.hvol, x, part);
+  else
+    k_dhpsi<false><<<g, HX * HY, 0, c->stream>>>(in, out, a, scale, c->gs.nblk, c->g.hvol, nullptr, nullptr);
   SB_LAUNCH_CHECK("k_dhpsi");
-  return SB200_OK;
-}
-
-// up to three per-orbital dot products into gs.d_dots[o][0..2] (times hvol)
-int gs_dots(sb200_ctx* c, int ndot, const double* x0, const double* y0, const double* x1 = nullptr,
-            const double* y1 = nullptr, const double* x2 = nullptr, const double* y2 = nullptr) {
-  GSState& s = c->gs;
-  DotArgs d;
-  d.npts = c->g.npts;
-  d.nblk = s.nblk;
-  d.ndot = ndot;
-  d.x0 = x0;
-  d.y0 = y0;
-  d.x1 = x1;
-  d.y1 = y1;
-  d.x2 = x2;
-  d.y2 = y2;
-  d.part = s.d_part;
-  dim3 g(s.nblk, c->orb.norb);
-  k_dots<<<g, RT, 0, c->stream>>>(d);
-  SB_LAUNCH_CHECK("k_dots");
-  k_dots_final<<<(c->orb.norb + 127) / 128, 128, 0, c->stream>>>(s.d_part, c->orb.norb, s.nblk, c->g.hvol,
-                                                                  s.d_dots);
-  SB_LAUNCH_CHECK("k_dots_final");
-  return SB200_OK;
-}
-
-int gs_scalars(sb200_ctx* c, int stage, int iter) {
-  k_cg_scalars<<<(c->orb.norb + 127) / 128, 128, 0, c->stream>>>(c->gs.d_coef, c->gs.d_dots, c->orb.norb, stage,
-                                                                  iter);
-  SB_LAUNCH_CHECK("k_cg_scalars");
-  return SB200_OK;
-}
-
-int gs_update(sb200_ctx* c, int op, double* a, double* b = nullptr, double* cc = nullptr, double* d = nullptr) {
-  UpdArgs u;
-  u.npts = c->g.npts;
-  u.n = c->gs.n;
-  u.op = op;
-  u.coef = c->gs.d_coef;
-  u.a = a;
-  u.b = b;
-  u.c = cc;
-  u.d = d;
-  k_cg_update<<<gridsz(u.n), 256, 0, c->stream>>>(u);
-  SB_LAUNCH_CHECK("k_cg_update");
   return SB200_OK;
 }
 
@@ -830,12 +989,6 @@ int gs_relayout(sb200_ctx* c, const double* src, double* dst, int norb, bool to_
                                                                  g.is[1] - g.is_array[1], g.is[2] - g.is_array[2],
                                                                  norb, to_ref ? 1 : 0);
   SB_LAUNCH_CHECK("k_relayout_real");
-  return SB200_OK;
-}
-
-int gs_axpy(sb200_ctx* c, double* y, const double* x, double a, long n) {
-  k_axpy<<<gridsz(n), 256, 0, c->stream>>>(y, x, a, n);
-  SB_LAUNCH_CHECK("k_axpy");
   return SB200_OK;
 }
 
@@ -1016,49 +1169,61 @@ int sb200_gscg(sb200_ctx* c, double* psi, int ncg, int precondition, double alph
   double* w = c->gs.d_work;
   double *xk = w, *hxk = w + n, *pk = w + 2 * n, *gk = w + 3 * n, *pre = w + 4 * n, *pko = w + 5 * n,
          *hwf = w + 6 * n;
-  SB_CUDA(cudaMemsetAsync(w, 0, sizeof(double) * 7 * n, c->stream));
-  SB_CUDA(cudaMemcpyAsync(xk, psi, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-  TRY_GS(gs_hpsi(c, xk, hxk));
-  TRY_GS(gs_dots(c, 1, xk, hxk));
-  TRY_GS(gs_scalars(c, 0, 0));
+  const int norb = c->orb.norb, nblk = c->gs.nblk;
+  const dim3 grid(nblk, norb), hg = dhpsi_grid(c);
+  const int nh = (int)(hg.x * hg.y);
+  // partial sums: <dir|g>, <x|pk>, <pko|pko>, the two of H, the two of the rotated x
+  const size_t ob = (size_t)norb * nblk;
+  double *p_xp = c->gs.d_part, *p_pp = p_xp + ob, *p_x = p_pp + ob, *p_h = p_x + 2 * ob, *p_gg = p_h + 2 * (size_t)norb * nh;
+  CgArgs a;
+  a.npts = c->g.npts;
+  a.nx = c->g.nx;
+  a.ny = c->g.ny;
+  a.nz = c->g.nz;
+  a.periodic = c->g.periodic;
+  a.hz = dhpsi_hz(c);
+  a.hvol = c->g.hvol;
+  a.state = c->gs.d_coef;
+  const double h0 = c->g.hgs[0], h1 = c->g.hgs[1], h2 = c->g.hgs[2];
+  const double omega_d = 2.0 * (1.0 - alpha_pre) /
+                         (-0.5 * ((-2.0) / (h0 * h0) + (-2.0) / (h1 * h1) + (-2.0) / (h2 * h2)));
+  const double* x = psi;  // the first iteration reads psi, later ones the rotated xk
+  TRY_GS(gs_hpsi(c, x, hxk, nullptr, x, p_h));
   for (int iter = 1; iter <= ncg; ++iter) {
-    TRY_GS(gs_update(c, U_GK, gk, hxk, xk));
-    const double* g_for_p = gk;
-    if (precondition == SB200_PRECOND_LOWPASS) {
-      TRY_GS(gs_precond(c, gk, pre, alpha_pre));
-      TRY_GS(gs_dots(c, 1, pre, gk));
-      g_for_p = pre;
-    } else if (precondition == SB200_PRECOND_LEARNED) {
-      TRY_GS(learned_precond_apply(c, gk, xk, pre));
-      TRY_GS(gs_dots(c, 1, pre, gk));
-      g_for_p = pre;
-    } else {
-      TRY_GS(gs_dots(c, 1, gk, gk));
+    const double* prev = iter == 1 ? p_h : p_x;
+    const int nprev = iter == 1 ? nh : nblk;
+    double* keep = iter == 1 ? nullptr : psi;
+    double* dir = precondition == SB200_PRECOND_LEARNED ? gk : pre;
+    if (precondition == SB200_PRECOND_LOWPASS)
+      k_cg_gradient<true><<<hg, HX * HY, 0, c->stream>>>(a, x, hxk, prev, nprev, keep, dir, 1.0 / (h0 * h0),
+                                                         1.0 / (h1 * h1), 1.0 / (h2 * h2), omega_d, p_gg);
+    else
+      k_cg_gradient<false><<<hg, HX * HY, 0, c->stream>>>(a, x, hxk, prev, nprev, keep, dir, 1.0, 1.0, 1.0, 0.0,
+                                                          p_gg);
+    SB_LAUNCH_CHECK("k_cg_gradient");
+    int ngg = nh;
+    if (precondition == SB200_PRECOND_LEARNED) {
+      ngg = nblk;
+      TRY_GS(learned_precond_apply(c, gk, x, pre));
+      k_cg_dot<<<grid, RT, 0, c->stream>>>(a, pre, gk, p_gg);
+      SB_LAUNCH_CHECK("k_cg_dot");
+      dir = pre;
     }
     // the network direction is not a fixed linear preconditioner: with it the
     // conjugation restarts every iteration (uk = 0, as in the first iteration)
-    TRY_GS(gs_scalars(c, 1, precondition == SB200_PRECOND_LEARNED ? 1 : iter));
-    TRY_GS(gs_update(c, U_PK, pk, (double*)g_for_p));
-    TRY_GS(gs_dots(c, 1, xk, pk));
-    TRY_GS(gs_scalars(c, 2, iter));
-    TRY_GS(gs_update(c, U_PKO, pko, pk, xk));
-    TRY_GS(gs_dots(c, 1, pko, pko));
-    TRY_GS(gs_scalars(c, 3, iter));
-    TRY_GS(gs_update(c, U_SCALE, pko));
-    TRY_GS(gs_hpsi(c, pko, hwf));
-    TRY_GS(gs_dots(c, 2, xk, hwf, pko, hwf));
-    TRY_GS(gs_scalars(c, 4, iter));
-    TRY_GS(gs_update(c, U_XH, xk, pko, hxk, hwf));
-    TRY_GS(gs_dots(c, 2, xk, hxk, xk, xk));
-    TRY_GS(gs_scalars(c, 5, iter));
-    TRY_GS(gs_update(c, U_PSI, psi, xk));
+    const int restart = iter == 1 || precondition == SB200_PRECOND_LEARNED;
+    k_cg_direction<<<grid, RT, 0, c->stream>>>(a, dir, x, p_gg, ngg, iter, restart, pk, p_xp);
+    SB_LAUNCH_CHECK("k_cg_direction");
+    k_cg_orthogonal<<<grid, RT, 0, c->stream>>>(a, pk, x, p_xp, pko, p_pp);
+    SB_LAUNCH_CHECK("k_cg_orthogonal");
+    TRY_GS(gs_hpsi(c, pko, hwf, p_pp, x, p_h));
+    k_cg_rotate<<<grid, RT, 0, c->stream>>>(a, x, xk, hxk, pko, hwf, p_pp, p_h, nh, p_x);
+    SB_LAUNCH_CHECK("k_cg_rotate");
+    x = xk;
   }
-  if (esp) {
-    std::vector<double> cf((size_t)c->orb.norb * CG_NC);
-    SB_CUDA(cudaMemcpyAsync(cf.data(), c->gs.d_coef, cf.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    SB_CUDA(cudaStreamSynchronize(c->stream));
-    for (int o = 0; o < c->orb.norb; ++o) esp[o] = cf[(size_t)o * CG_NC + CG_XKHXK] / cf[(size_t)o * CG_NC + CG_XKXK];
-  }
+  k_cg_end<<<grid, RT, 0, c->stream>>>(a, x, p_x, nblk, psi, c->gs.d_dots);
+  SB_LAUNCH_CHECK("k_cg_end");
+  if (esp) SB_CUDA(cudaMemcpyAsync(esp, c->gs.d_dots, norb * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   SB_CUDA(cudaStreamSynchronize(c->stream));
   return SB200_OK;
 }

@@ -87,6 +87,12 @@ struct PPInfo {
   double2* d_pair_ph = nullptr; // [nk_phase][npair]
   int* d_pair_pt = nullptr;     // [npair] grid point of the pair
   int* d_apj = nullptr;         // [totpts] pair of each flat sphere point
+  // the cluster-resident fused step's tables (sb200_orbital_any.cu)
+  int* d_pst = nullptr;         // [natom][nz + 1] first flat sphere point at or above each plane
+  int* d_ppl = nullptr;         // [nz + 1] first pair at or above each plane
+  double* d_uv4 = nullptr;      // [totpts][4] uV of the atom's projectors
+  double* d_pair_r = nullptr;   // [npair][3] coordinates of each pair's sphere point
+  std::vector<int> h_ppl;       // host copy of d_ppl
   // the register-blocked fused step's tables in its shared-memory layout (16^3 grids)
   int blk_tpad = 0;
   double* d_blk_uv = nullptr;   // [4][blk_tpad]
@@ -115,15 +121,16 @@ struct RTBuffers {
 };
 
 // ground-state (real orbital) work state, sb200_gs.cu
-constexpr int CG_NC = 12;  // per-orbital CG coefficients
-enum { CG_XKHXK = 0, CG_GKGK, CG_UK, CG_ZS, CG_SUM, CG_CX, CG_CP, CG_XKXK };
+constexpr int CG_NC = 4;  // per-orbital CG scalars kept between launches
+enum { CG_XKHXK = 0, CG_GG0, CG_GG1 };
 struct GSState {
   long n = 0;         // npts * norb of the buffers below
   int norb = 0, nblk = 0;
+  size_t npart = 0, nproj = 0;  // capacities of d_part and d_proj
   bool have_work = false;
   double* d_proj = nullptr;   // [norb][nlma] real projections
-  double* d_part = nullptr;   // [norb][nblk][3] dot partials
-  double* d_dots = nullptr;   // [norb][3]
+  double* d_part = nullptr;   // partial sums of the CG's launches
+  double* d_dots = nullptr;   // [norb]
   double* d_coef = nullptr;   // [norb][CG_NC]
   double* d_work = nullptr;   // 7 orbital blocks for the CG
   double* d_gram = nullptr;   // Gram partials
@@ -165,6 +172,10 @@ struct sb200_ctx {
   void* d_stage = nullptr;      // relayout staging
   size_t stage_bytes = 0;
   bool vloc_set = false;
+  int any_C = -1;              // cluster size of the fused step of general periodic grids (0: does not apply,
+                               // -1: to be chosen at the next step)
+  int any_resident = 0;        // its clusters at work at a time
+  int any_smem_cap = 0, any_static = 0;  // dynamic shared memory one of its CTAs can take, its static part
   int stencil_variant = 1;     // 0: per-point reference kernel, 1: tiled 2.5-D sweep
   int orbital_variant = 4;     // 16^3 periodic grids: 4 fused Taylor step with register blocking (when its
                                // tables fit, else form 2), 2 fused step with the KB tables staged in shared memory
@@ -177,6 +188,7 @@ struct sb200_ctx {
                                // stencil (1), or one warp per atom between the terms (0)
   int blk_prefetch = 1;        // blocked fused step: each CTA prefetches the orbital one wave ahead into L2
   int tma_variant = 1;         // tiled hpsi fed by tensor copies where it applies (0: register-prefetch sweep)
+  bool sweep_asked = false;    // the environment names a sweep: the cluster-resident step stays off
   // optional per-kernel-class device timing (sb200_set_timing)
   bool timing = false;
   std::vector<cudaEvent_t> ev;  // pairs (start, stop)
@@ -300,6 +312,10 @@ int launch_energy_parts(sb200_ctx* c, const double2* psi, const double2* h, cons
 bool step_orbital_applies(const sb200_ctx* c, int n_hamil);                  // sb200_orbital.cu
 int launch_step_orbital(sb200_ctx* c, const double2* in, double2* out, const double2* zc, int n_hamil,
                         bool with_obs);
+// the fused step of general periodic grids (sb200_orbital_any.cu)
+bool step_any_applies(sb200_ctx* c, int n_hamil);
+int launch_step_any(sb200_ctx* c, const double2* in, double2* out, const double2* zc, int n_hamil, bool with_obs,
+                    bool hmode);
 int launch_observables(sb200_ctx* c, const double2* psi);
 struct KickArgs {
   double e, ep[3], h[3], c0[3];  // e_impulse, direction, spacing, coordinate offset per axis
