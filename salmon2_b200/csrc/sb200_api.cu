@@ -2,6 +2,7 @@
 // hpsi / taylor / observable entry points and the CUDA-graph time loop.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -78,6 +79,7 @@ int ensure_stage(sb200_ctx* c, size_t bytes) {
 
 // (re)allocate work buffers that depend on grid x orbitals x projectors
 int ensure_work(sb200_ctx* c) {
+  c->any_C = -1;  // the fused step's shape is chosen anew
   if (!c->g.set || !c->orb.set) return SB200_OK;
   dfree(c->d_proj);
   dfree(c->d_jw);
@@ -138,6 +140,10 @@ void free_pp(PPInfo& p) {
   dfree(p.d_pair_uv);
   dfree(p.d_pair_fp);
   dfree(p.d_pair_ph);
+  dfree(p.d_pst);
+  dfree(p.d_ppl);
+  dfree(p.d_uv4);
+  dfree(p.d_pair_r);
   dfree(p.d_blk_uv);
   dfree(p.d_blk_r);
   dfree(p.d_blk_sap);
@@ -226,6 +232,10 @@ int issue_taylor(sb200_ctx* c, double2* tin, double2* tout, double2* work, const
                  bool last_with_obs = false) {
   if (step_orbital_applies(c, n_hamil)) {  // all terms in one launch, observables fused
     TIMED(c, SB200_KIND_HPSI, launch_step_orbital(c, tin, tout, zc, n_hamil, last_with_obs));
+    return SB200_OK;
+  }
+  if (step_any_applies(c, n_hamil)) {
+    TIMED(c, SB200_KIND_HPSI, launch_step_any(c, tin, tout, zc, n_hamil, last_with_obs, false));
     return SB200_OK;
   }
   const bool orbital = orbital_kernel_applies(c);
@@ -347,7 +357,7 @@ int issue_rt_step(sb200_ctx* c, double2* in, double2* out, double2* work, const 
     TRY(issue_taylor(c, in, out, work, zc, n_hamil));
     TIMED(c, SB200_KIND_POTENTIAL, launch_aetrs_vloc(c));
     if (c->g.periodic) TIMED(c, SB200_KIND_PREP, launch_prep_k(c, c->rt.d_Ac_ext, 3, -1, c->d_kcoef, true));
-    if (orbital_kernel_applies(c) && c->gs_interval < 1) {
+    if ((orbital_kernel_applies(c) || step_any_applies(c, n_hamil)) && c->gs_interval < 1) {
       TRY(issue_taylor(c, out, in, work, zc, n_hamil, true));
       TIMED(c, SB200_KIND_FINAL, launch_finalize(c, -1, 0, trans_longi, dt, -1, true));
       return scf_rt_issue(c, in);
@@ -369,7 +379,7 @@ int issue_rt_step(sb200_ctx* c, double2* in, double2* out, double2* work, const 
     TRY(scf_pc_potential(c, out, c->d_pc_v, c->d_pc_v + nv));
     SB_CUDA(cudaMemcpyAsync(in, c->d_pc_psi, nb * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
   }
-  if (orbital_kernel_applies(c) && c->gs_interval < 1) {  // observables fused into the last Taylor term
+  if ((orbital_kernel_applies(c) || step_any_applies(c, n_hamil)) && c->gs_interval < 1) {  // observables fused into the last Taylor term
     TRY(issue_taylor(c, in, out, work, zc, n_hamil, true));
     TIMED(c, SB200_KIND_FINAL, launch_finalize(c, -1, 0, trans_longi, dt, -1, true));
     return scf_rt_issue(c, out);
@@ -418,7 +428,10 @@ int sb200_ctx_create(int device, sb200_ctx** out) {
   if (const char* v = getenv("SB200_BLK_DEPTH")) c->blk_depth = (v[0] == '4') ? 4 : 2;
   if (const char* v = getenv("SB200_BLK_SPLIT")) c->blk_split = (v[0] == '0') ? 0 : 1;
   if (const char* v = getenv("SB200_BLK_PREFETCH")) c->blk_prefetch = (v[0] == '0') ? 0 : 1;
-  if (const char* v = getenv("SB200_TMA")) c->tma_variant = (v[0] == 'o' && v[1] == 'f') ? 0 : 1;
+  if (const char* v = getenv("SB200_TMA")) {  // asks for one of the two sweeps
+    c->tma_variant = (v[0] == 'o' && v[1] == 'f') ? 0 : 1;
+    c->sweep_asked = true;
+  }
   int r = dalloc(&c->d_result, 24);  // results [0, 8), staged A [8, 11), shard sums [16, 23)
   if (r == SB200_OK) r = dalloc(&c->rt.d_step, 1);
   if (r == SB200_OK) r = dalloc(&c->d_err, 1);
@@ -683,34 +696,41 @@ int sb200_set_pp(sb200_ctx* c, int natom, int nps, int nlma, const int* mps, con
   }
   std::vector<int> pt_lin(tot);
   std::vector<double> pt_r(3 * (size_t)tot);
-  for (int a = 0; a < natom; ++a)
+  // each atom's sphere points in grid order (src: the caller's index): the part
+  // of an atom in a range of planes is one run, and gathers go up in memory
+  std::vector<int> src(tot), lin0;
+  for (int a = 0; a < natom; ++a) {
+    lin0.resize(hmps[a]);
     for (int j = 0; j < hmps[a]; ++j) {
       int ic[3];
       for (int d = 0; d < 3; ++d) {
         ic[d] = jxyz[d + 3L * (j + (long)nps * a)];
         if (ic[d] < g.is[d] || ic[d] > g.ie[d])  // host-side bounds check of every table index
           return set_error(SB200_ERR_BAD_SHAPE, "jxyz point outside the grid interior");
-        pt_r[3L * (atom_start[a] + j) + d] = rxyz[d + 3L * (j + (long)nps * a)];
       }
-      pt_lin[atom_start[a] + j] =
-          (ic[0] - g.is[0]) + g.nx * ((ic[1] - g.is[1]) + (long)g.ny * (ic[2] - g.is[2]));
+      lin0[j] = (ic[0] - g.is[0]) + g.nx * ((ic[1] - g.is[1]) + (long)g.ny * (ic[2] - g.is[2]));
+      src[atom_start[a] + j] = j;
     }
-  // inverse map: point -> (ilma, flat point, uv) entries in ilma order
-  std::vector<std::vector<int>> ent_of_point;
-  std::vector<int> map(g.npts, -1), vi_pt;
-  std::vector<int> cnt;
-  for (int l = 0; l < nlma; ++l) {
-    const int a = ia_tbl[l] - 1;
+    std::stable_sort(src.begin() + atom_start[a], src.begin() + atom_start[a] + hmps[a],
+                     [&](int i, int j) { return lin0[i] < lin0[j]; });
     for (int j = 0; j < hmps[a]; ++j) {
-      const int p = pt_lin[atom_start[a] + j];
-      if (map[p] < 0) {
-        map[p] = (int)vi_pt.size();
-        vi_pt.push_back(p);
-        cnt.push_back(0);
-      }
-      cnt[map[p]] += 1;
+      const int fp = atom_start[a] + j, js = src[fp];
+      pt_lin[fp] = lin0[js];
+      for (int d = 0; d < 3; ++d) pt_r[3L * fp + d] = rxyz[d + 3L * (js + (long)nps * a)];
     }
   }
+  // inverse map: point -> (ilma, flat point, uv) entries in ilma order
+  std::vector<int> map(g.npts, -1), vi_pt, cnt, npt(g.npts, 0);
+  for (int l = 0; l < nlma; ++l) {
+    const int a = ia_tbl[l] - 1;
+    for (int j = 0; j < hmps[a]; ++j) npt[pt_lin[atom_start[a] + j]] += 1;
+  }
+  for (long q = 0; q < g.npts; ++q)
+    if (npt[q] > 0) {  // points in grid order
+      map[q] = (int)vi_pt.size();
+      vi_pt.push_back((int)q);
+      cnt.push_back(npt[q]);
+    }
   const int nvi = (int)vi_pt.size();
   std::vector<int> vi_start(nvi + 1, 0);
   for (int v = 0; v < nvi; ++v) vi_start[v + 1] = vi_start[v] + cnt[v];
@@ -725,12 +745,14 @@ int sb200_set_pp(sb200_ctx* c, int natom, int nps, int nlma, const int* mps, con
       const int e = fill[v]++;
       ent_lma[e] = l;
       ent_pt[e] = fp;
-      ent_uv[e] = uv[j + (long)nps * l];
+      ent_uv[e] = uv[src[fp] + (long)nps * l];
     }
   }
   std::vector<double> huv((size_t)nlma * (nps > 0 ? nps : 1), 0.0);
-  for (int l = 0; l < nlma; ++l)
-    for (int j = 0; j < nps; ++j) huv[(size_t)l * nps + j] = uv[j + (long)nps * l];
+  for (int l = 0; l < nlma; ++l) {
+    const int a = ia_tbl[l] - 1;
+    for (int j = 0; j < hmps[a]; ++j) huv[(size_t)l * nps + j] = uv[src[atom_start[a] + j] + (long)nps * l];
+  }
   std::vector<double> hrinv(rinv_uvu, rinv_uvu + nlma);
   PPInfo& p = c->pp;
   p.natom = natom;
@@ -815,6 +837,29 @@ int sb200_set_pp(sb200_ctx* c, int natom, int nps, int nlma, const int* mps, con
     TRY(upload(&p.d_pair_uv, pair_uv));
     TRY(upload(&p.d_pair_fp, pair_fp));
     TRY(blk_build_tables(c, pt_lin, apj, huv, pt_r, atom_start, hmps, lma_start, nproj));
+    if (g.periodic) {  // the cluster-resident fused step: runs of each atom and of the pairs by plane
+      const int plane = g.nx * g.ny;
+      std::vector<int> pst((size_t)natom * (g.nz + 1));
+      std::vector<double> uv4(4 * (size_t)(tot > 0 ? tot : 1), 0.0);
+      for (int at = 0; at < natom; ++at) {
+        const auto b0 = pt_lin.begin() + atom_start[at], b1 = b0 + hmps[at];
+        for (int z = 0; z <= g.nz; ++z)
+          pst[(size_t)at * (g.nz + 1) + z] = (int)(std::lower_bound(b0, b1, z * plane) - pt_lin.begin());
+        for (int j = 0; j < hmps[at]; ++j)
+          for (int q = 0; q < nproj[at]; ++q)
+            uv4[4 * (size_t)(atom_start[at] + j) + q] = huv[(size_t)(lma_start[at] + q) * nps + j];
+      }
+      p.h_ppl.resize(g.nz + 1);
+      for (int z = 0; z <= g.nz; ++z)
+        p.h_ppl[z] = (int)(std::lower_bound(pair_pt.begin(), pair_pt.end(), z * plane) - pair_pt.begin());
+      std::vector<double> pair_r(3 * pair_fp.size());
+      for (size_t i = 0; i < pair_fp.size(); ++i)
+        for (int d = 0; d < 3; ++d) pair_r[3 * i + d] = pt_r[3 * (size_t)pair_fp[i] + d];
+      TRY(upload(&p.d_pair_r, pair_r));
+      TRY(upload(&p.d_pst, pst));
+      TRY(upload(&p.d_uv4, uv4));
+      TRY(upload(&p.d_ppl, p.h_ppl));
+    }
     TRY(dalloc(&p.d_pair_ph, (size_t)p.nk_phase * (p.npair > 0 ? p.npair : 1)));
     if (!g.periodic) {  // isolated: exp(i 0.r) = 1
       std::vector<double2> one(p.npair > 0 ? p.npair : 1, make_double2(1.0, 0.0));
@@ -1042,6 +1087,10 @@ int sb200_hpsi(sb200_ctx* c, const double* tpsi, double* htpsi) {
   TRY(require_ready(c));
   if (!tpsi || !htpsi || tpsi == htpsi) return set_error(SB200_ERR_INVALID_ARG, "tpsi/htpsi null or aliased");
   DeviceGuard dg(c->device);
+  if (step_any_applies(c, 1)) {  // projections and stencil in one launch
+    TIMED(c, SB200_KIND_HPSI, launch_step_any(c, (const double2*)tpsi, (double2*)htpsi, nullptr, 1, false, true));
+    return SB200_OK;
+  }
   TIMED(c, SB200_KIND_PROJECT, launch_project(c, (const double2*)tpsi, c->d_proj));
   HpsiLaunch L;
   L.in = (const double2*)tpsi;
