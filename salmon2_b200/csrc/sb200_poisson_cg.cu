@@ -39,6 +39,12 @@
 // word that releases the other blocks and the context's error flag, which the
 // host turns into SB200_ERR_TIMEOUT.  The two-launch form stays for
 // SB200_PCG_PERSISTENT=0 and where a cooperative launch cannot be captured.
+//
+// Grids whose boxes fit one CTA each (up to about 70^3) take k_pcg_box instead:
+// every vector stays in registers and shared memory for the whole solve, only
+// the Laplacian of the residual and two partial sums go through L2, and the
+// recurrences of Chronopoulos and Gear (J. Comput. Appl. Math. 25, 1989) need
+// one grid barrier per iteration instead of two.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -226,8 +232,8 @@ __device__ __forceinline__ bool pole_point(const PArgs& a, int pole, long p, int
 // moments r^l Ylm rho hvol about the pole's centre.  Grid (nchunk, npole).
 template <int KIND>
 __global__ void __launch_bounds__(PT) k_pcg_pole_sum(PArgs a) {
-  __shared__ double red[PT / 32 + 1];
   constexpr int NV = KIND == 0 ? 4 : NLM_MAX;
+  __shared__ double red[NV][PT / 32];
   const int pole = blockIdx.y;
   double acc[NV];
 #pragma unroll
@@ -263,36 +269,45 @@ __global__ void __launch_bounds__(PT) k_pcg_pole_sum(PArgs a) {
       }
     }
   }
+  // butterfly in the warp, then the warps in order, all values behind one barrier
   double* out = a.psum + ((long)pole * a.nchunk + blockIdx.x) * NLM_MAX;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    const double s = block_sum(acc[v], red);
-    if (threadIdx.x == 0) out[v] = s;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
+    if ((threadIdx.x & 31) == 0) red[v][threadIdx.x >> 5] = acc[v];
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double s = red[threadIdx.x][0];
+    for (int w = 1; w < PT / 32; ++w) s += red[threadIdx.x][w];
+    out[threadIdx.x] = s;
   }
 }
 
-// pole entries from the partial sums (one thread per pole; chunks in order).
-// KIND 0: centroid and itrho of the layout-3 cells; KIND 1: rholm.
+// pole entries from the partial sums: a block per pole, 32 lanes over the values
+// x 8 slices of the chunks, the slices added in order (a thread per pole took 21
+// us for 8 poles).  KIND 0: centroid and itrho of the layout-3 cells; KIND 1: rholm.
 template <int KIND>
-__global__ void k_pcg_pole_reduce(PArgs a) {
-  const int pole = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pole >= a.npole) return;
+__global__ void __launch_bounds__(256) k_pcg_pole_reduce(PArgs a) {
+  __shared__ double red[8][32];
+  const int pole = blockIdx.x, v = threadIdx.x, nv = KIND == 0 ? 4 : a.nlm;
   double* pe = a.pole + (long)pole * POLE_W;
   const double* ps = a.psum + (long)pole * a.nchunk * NLM_MAX;
+  double s = 0.0;
+  if (v < nv)
+    for (int c = threadIdx.y; c < a.nchunk; c += 8) s += ps[(long)c * NLM_MAX + v];
+  red[threadIdx.y][v] = s;
+  __syncthreads();
+  if (threadIdx.y != 0) return;
+  for (int y = 1; y < 8; ++y) s += red[y][v];
   if (KIND == 0) {
-    double s[4] = {0, 0, 0, 0};
-    for (int c = 0; c < a.nchunk; ++c)
-      for (int v = 0; v < 4; ++v) s[v] += ps[(long)c * NLM_MAX + v];
-    const bool on = s[3] * a.hvol >= 1e-12;
-    for (int d = 0; d < 3; ++d) pe[d] = on ? s[d] / s[3] : 0.0;
-    pe[3] = on ? 1.0 : 0.0;
-  } else {
-    for (int lm = 0; lm < NLM_MAX; ++lm) {
-      double s = 0.0;
-      if (lm < a.nlm)
-        for (int c = 0; c < a.nchunk; ++c) s += ps[(long)c * NLM_MAX + lm];
-      pe[4 + lm] = s;
-    }
+    const double q = __shfl_sync(0xffffffffu, s, 3);
+    const bool on = q * a.hvol >= 1e-12;
+    if (v < 3) pe[v] = on ? s / q : 0.0;
+    if (v == 3) pe[3] = on ? 1.0 : 0.0;
+  } else if (v < NLM_MAX) {
+    pe[4 + v] = s;  // zero past nlm
   }
 }
 
@@ -627,6 +642,208 @@ __global__ void __launch_bounds__(PTP, 2) k_pcg_solve(PArgs a) {
   }
 }
 
+// ---- CG with every vector on chip ----------------------------------------------
+// One CTA per box of the grid.  The box's p, x, s = lap p and w = lap r live in
+// registers, its residual r in shared memory with a 4-point halo in the six
+// directions (a dense box of (b + 8)^3, zero outside the grid).  Per iteration a
+// CTA reads w at its halo points from L2, repeats there the two updates its
+// neighbours make (s = w + beta s, r -= alpha s), so no halo of r is exchanged,
+// makes them at its own points, forms w = lap r from shared memory, publishes it
+// (two buffers in turn: a neighbour may still read the last one), and adds
+// (r, r) and (w, r) to the sums of the one grid barrier:
+//   beta = (r, r) / (r, r)_old,  alpha = (r, r) / ((w, r) - beta (r, r) / alpha_old)
+// which is the reference's (r, r) / (r, lap p).  The convergence test is that of
+// poisson_isolated_cg on the same residual.  64^3 in 144 boxes: 50 loads a point
+// through L1 / L2 and two barriers took 13.5 us an iteration.
+constexpr int BXT = 512;
+struct Boxes {
+  int g[3] = {0, 0, 0};  // boxes per axis (0: the form does not apply)
+  size_t smem = 0;
+  int own = 0, halo = 0; // largest counts of a box
+};
+
+template <int MO, int MH>
+__global__ void __launch_bounds__(BXT, 1) k_pcg_box(PArgs a, int gx, int gy, int gz) {
+  extern __shared__ double r[];
+  __shared__ double red[2][BXT / 32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nb = (int)gridDim.x;
+  const int jx = blockIdx.x % gx, jy = (blockIdx.x / gx) % gy, jz = blockIdx.x / (gx * gy);
+  const int x0 = jx * a.nx / gx, y0 = jy * a.ny / gy, z0 = jz * a.nz / gz;
+  const int bx = (jx + 1) * a.nx / gx - x0, by = (jy + 1) * a.ny / gy - y0, bz = (jz + 1) * a.nz / gz - z0;
+  const int ex = bx + 2 * HALO, ey = by + 2 * HALO, sy = ex, sz = ex * ey;
+  const int nown = bx * by * bz;
+  const int fx = by * bz, fy = bx * bz, fz = bx * by, nhalo = 2 * HALO * (fx + fy + fz);
+  auto eidx = [&](int x, int y, int z) { return x + HALO + sy * (y + HALO) + sz * (z + HALO); };
+  auto cidx = [&](int x, int y, int z) { return (int)padi(a, x0 + x, y0 + y, z0 + z); };
+  int eo[MO], co[MO], eh[MH], ch[MH];
+  double p[MO], x[MO], w[MO], s[MO], sh[MH];
+#pragma unroll
+  for (int i = 0; i < MO; ++i) {
+    const int q = t + i * BXT;
+    eo[i] = -1;
+    co[i] = 0;
+    p[i] = s[i] = x[i] = w[i] = 0.0;
+    if (q < nown) {
+      const int lx = q % bx, ly = (q / bx) % by, lz = q / (bx * by);
+      eo[i] = eidx(lx, ly, lz);
+      co[i] = cidx(lx, ly, lz);
+      r[eo[i]] = a.zk[co[i]];
+      x[i] = a.vh[(x0 + lx) + (long)a.nx * ((y0 + ly) + (long)a.ny * (z0 + lz))];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MH; ++i) {
+    int q = t + i * BXT;
+    eh[i] = -1;
+    ch[i] = 0;
+    sh[i] = 0.0;
+    if (q < nhalo) {
+      int lx, ly, lz;
+      if (q < 2 * HALO * fx) {
+        const int h = q % (2 * HALO), u = q / (2 * HALO);
+        lx = h < HALO ? h - HALO : bx + h - HALO;
+        ly = u % by;
+        lz = u / by;
+      } else if ((q -= 2 * HALO * fx) < 2 * HALO * fy) {
+        lx = q % bx;
+        const int u = q / bx, h = u % (2 * HALO);
+        ly = h < HALO ? h - HALO : by + h - HALO;
+        lz = u / (2 * HALO);
+      } else {
+        q -= 2 * HALO * fy;
+        lx = q % bx;
+        const int u = q / bx, h = u / by;
+        ly = u % by;
+        lz = h < HALO ? h - HALO : bz + h - HALO;
+      }
+      // at most 4 points past the grid: inside the padding, where zk and w are zero
+      eh[i] = eidx(lx, ly, lz);
+      ch[i] = cidx(lx, ly, lz);
+      r[eh[i]] = a.zk[ch[i]];
+    }
+  }
+  __syncthreads();
+  auto laplacian = [&](int e) {
+    const double* f = r + e;
+    double tx = a.lapt[0] * (f[1] + f[-1]), ty = a.lapt[4] * (f[sy] + f[-sy]), tz = a.lapt[8] * (f[sz] + f[-sz]);
+#pragma unroll
+    for (int k = 1; k < HALO; ++k) {
+      tx = fma(a.lapt[k], f[k + 1] + f[-k - 1], tx);
+      ty = fma(a.lapt[4 + k], f[(k + 1) * sy] + f[-(k + 1) * sy], ty);
+      tz = fma(a.lapt[8 + k], f[(k + 1) * sz] + f[-(k + 1) * sz], tz);
+    }
+    return fma(-2.0 * a.lap0, f[0], (tx + ty) + tz);
+  };
+  // sums of the two values over the block, left in part[par][block]; then the
+  // grid barrier and the sums over the blocks, in block order
+  unsigned int target = 0u;
+  double tot[2];
+  auto block2 = [&](double v0, double v1) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+      v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    __syncthreads();
+    if (lane == 0) {
+      red[0][warp] = v0;
+      red[1][warp] = v1;
+    }
+    __syncthreads();
+    double u0 = 0.0, u1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < BXT / 32; ++i) {
+      u0 += red[0][i];
+      u1 += red[1][i];
+    }
+    tot[0] = u0;
+    tot[1] = u1;
+  };
+  auto exchange = [&](double v0, double v1, int par) -> bool {
+    block2(v0, v1);
+    double2* part = (double2*)a.part + par * nb;
+    if (t == 0) part[blockIdx.x] = make_double2(tot[0], tot[1]);
+    if (!grid_barrier(a, target)) return false;
+    double2 v = make_double2(0.0, 0.0);
+    if (t < nb) v = __ldcg(part + t);  // at most one block per SM: nb < BXT
+    block2(v.x, v.y);
+    return true;
+  };
+  double rr = 0.0, wr = 0.0;
+#pragma unroll
+  for (int i = 0; i < MO; ++i)
+    if (eo[i] >= 0) {
+      w[i] = laplacian(eo[i]);
+      __stcg(a.pk[0] + co[i], w[i]);
+      wr = fma(w[i], r[eo[i]], wr);
+    }
+  if (!exchange(0.0, wr, 0)) return;
+  double gamma = a.sc[SC_SUM1] / a.hvol, beta = 0.0, alpha = gamma / tot[1];
+  double done = 0.0, iter = 0.0;
+  int it = 1;
+  for (; it <= a.maxiter; ++it) {
+    const double* wp = a.pk[(it + 1) & 1];
+    double* wn = a.pk[it & 1];
+    double hv[MH];
+#pragma unroll
+    for (int i = 0; i < MH; ++i) hv[i] = eh[i] >= 0 ? __ldcg(wp + ch[i]) : 0.0;
+    rr = 0.0;
+    wr = 0.0;
+#pragma unroll
+    for (int i = 0; i < MO; ++i)
+      if (eo[i] >= 0) {
+        const double rv = r[eo[i]];
+        p[i] = fma(beta, p[i], rv);
+        s[i] = fma(beta, s[i], w[i]);
+        x[i] = fma(alpha, p[i], x[i]);
+        const double rn = fma(-alpha, s[i], rv);
+        r[eo[i]] = rn;
+        rr = fma(rn, rn, rr);
+      }
+#pragma unroll
+    for (int i = 0; i < MH; ++i)
+      if (eh[i] >= 0) {
+        sh[i] = fma(beta, sh[i], hv[i]);
+        r[eh[i]] = fma(-alpha, sh[i], r[eh[i]]);
+      }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < MO; ++i)
+      if (eo[i] >= 0) {
+        w[i] = laplacian(eo[i]);
+        __stcg(wn + co[i], w[i]);
+        wr = fma(w[i], r[eo[i]], wr);
+      }
+    if (!exchange(rr, wr, it & 1)) return;
+    const double sum2 = tot[0] * a.hvol;
+    if (fabs(sum2) < a.threshold * (double)a.N) {
+      done = 1.0;
+      iter = (double)it;
+      break;
+    }
+    beta = tot[0] / gamma;
+    alpha = tot[0] / (tot[1] - beta * tot[0] / alpha);
+    gamma = tot[0];
+    if (it >= a.maxiter) {
+      done = 2.0;
+      iter = (double)(a.maxiter + 1);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MO; ++i) {
+    const int q = t + i * BXT;
+    if (q < nown)
+      a.vh[(x0 + q % bx) + (long)a.nx * ((y0 + (q / bx) % by) + (long)a.ny * (z0 + q / (bx * by)))] = x[i];
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    a.sc[SC_SUM1] = gamma * a.hvol;
+    a.sc[SC_CK] = beta;
+    a.sc[SC_DONE] = done;
+    a.sc[SC_ITER] = iter;
+    a.sc[SC_NEXT] = (double)(done == 1.0 ? it + 1 : it);
+  }
+}
+
 // Check of the grid barrier: `rounds` barriers over the solve's cooperative
 // grid.  With withhold != 0 block 0 leaves without arriving, so the other
 // blocks' bounded waits expire (about a second of SM clock) and set the abort
@@ -664,6 +881,7 @@ struct PcgState {
   cudaStream_t side = nullptr;  // captures the body of the conditional node
   int unroll = PCG_UNROLL;      // CG iterations per body of the conditional node
   int solve_grid = 0;           // blocks of k_pcg_solve (0: the two-launch form)
+  Boxes box;                    // boxes of k_pcg_box
 };
 
 PcgState* pcg_of(sb200_ctx* c) { return static_cast<PcgState*>(c->pcg); }
@@ -700,6 +918,71 @@ cudaError_t launch_coop(void (*kernel)(PArgs, Args...), int grid, cudaStream_t s
 }
 
 cudaError_t launch_solve(const PArgs& a, int grid, cudaStream_t st) { return launch_coop(k_pcg_solve, grid, st, a); }
+
+// own and halo points a thread of k_pcg_box can hold, by instantiation
+constexpr int BOX_MO[3] = {2, 4, 6}, BOX_MH[3] = {5, 8, 11};
+int box_which(const Boxes& b) {
+  for (int i = 0; i < 3; ++i)
+    if (b.own <= BOX_MO[i] * BXT && b.halo <= BOX_MH[i] * BXT) return i;
+  return -1;
+}
+const void* box_kernel(int which) {
+  return which == 0   ? (const void*)k_pcg_box<BOX_MO[0], BOX_MH[0]>
+         : which == 1 ? (const void*)k_pcg_box<BOX_MO[1], BOX_MH[1]>
+                      : (const void*)k_pcg_box<BOX_MO[2], BOX_MH[2]>;
+}
+
+cudaError_t launch_box(const PArgs& a, const Boxes& b, cudaStream_t st) {
+  const int nb = b.g[0] * b.g[1] * b.g[2];
+  int gx = b.g[0], gy = b.g[1], gz = b.g[2];
+  PArgs arg = a;
+  void* args[4] = {&arg, &gx, &gy, &gz};
+  return cudaLaunchCooperativeKernel(box_kernel(box_which(b)), dim3((unsigned)nb), dim3(BXT), args, b.smem, st);
+}
+
+// The boxes of k_pcg_box for the grid: no more than SMs (one CTA each), the
+// largest box's points plus a third of its halo points (a load and two
+// operations each against the 25-point sum) the smallest; none when a box does
+// not fit its CTA, or with SB200_PCG_PERSISTENT=0 or =rows (k_pcg_solve).
+Boxes boxes_for(int nx, int ny, int nz, int device) {
+  Boxes best, b;
+  if (const char* v = std::getenv("SB200_PCG_PERSISTENT"))
+    if (v[0] == '0' || v[0] == 'r') return best;
+  int sms = 0, optin = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
+    cudaGetLastError();
+    return best;
+  }
+  if (sms >= BXT) sms = BXT - 1;
+  double cost = 0.0;
+  for (int gx = 1; gx <= nx && gx <= sms; ++gx)
+    for (int gy = 1; gy <= ny && gx * gy <= sms; ++gy) {
+      const int gz = sms / (gx * gy) < nz ? sms / (gx * gy) : nz;
+      const int bx = (nx + gx - 1) / gx, by = (ny + gy - 1) / gy, bz = (nz + gz - 1) / gz;
+      b.g[0] = gx;
+      b.g[1] = gy;
+      b.g[2] = gz;
+      b.own = bx * by * bz;
+      b.halo = 2 * HALO * (by * bz + bx * bz + bx * by);
+      b.smem = (size_t)(bx + 2 * HALO) * (by + 2 * HALO) * (bz + 2 * HALO) * sizeof(double);
+      if (box_which(b) < 0 || b.smem + 1024 > (size_t)optin) continue;
+      const double w = b.own + b.halo / 3.0;
+      if (best.g[0] == 0 || w < cost) {
+        cost = w;
+        best = b;
+      }
+    }
+  if (best.g[0] == 0) return best;
+  const void* k = box_kernel(box_which(best));
+  int per_sm = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best.smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, BXT, best.smem) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    return Boxes();
+  }
+  return best;
+}
 
 // Blocks of the one-launch solve: at most two per SM (one with
 // SB200_PCG_SOLVE_BLOCKS_PER_SM=1) and no more than the points need, within
@@ -856,8 +1139,10 @@ int pcg_configure(sb200_ctx* c, int layout, int lmax, const double* rion, int na
     SB_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
     s->solve_grid = solve_grid_for(a.N, s->side, c->device);
   }
+  if (s->solve_grid > 0) s->box = boxes_for(nx, ny, nz, c->device);
   const int nblk = grid_blocks(a.N);
-  const long n_part = nblk > 2L * s->solve_grid ? nblk : 2L * s->solve_grid;  // k_pcg_solve: two partial arrays
+  long n_part = nblk > 2L * s->solve_grid ? nblk : 2L * s->solve_grid;  // k_pcg_solve: two partial arrays
+  if (n_part < 4L * BXT) n_part = 4L * BXT;  // k_pcg_box: two arrays of two sums a block
   const size_t b_pad = al(P * sizeof(double)), b_int = al(a.N * sizeof(double));
   const size_t b_part = al((size_t)n_part * sizeof(double)), b_sc = al(8 * sizeof(double) + sizeof(unsigned int) * 8);
   const size_t b_pole = al((size_t)a.npole * POLE_W * sizeof(double));
@@ -941,13 +1226,12 @@ int pcg_issue(sb200_ctx* c, const double* d_rho, double* d_vh, int* iterations) 
   cudaStream_t st = c->stream;
   const int gb = grid_blocks(a.N);
   const dim3 gpole(a.nchunk, a.npole);
-  const int gred = (a.npole + 127) / 128;
   if (a.layout == 3) {
     k_pcg_pole_sum<0><<<gpole, PT, 0, st>>>(a);
-    k_pcg_pole_reduce<0><<<gred, 128, 0, st>>>(a);
+    k_pcg_pole_reduce<0><<<a.npole, dim3(32, 8), 0, st>>>(a);
   }
   k_pcg_pole_sum<1><<<gpole, PT, 0, st>>>(a);
-  k_pcg_pole_reduce<1><<<gred, 128, 0, st>>>(a);
+  k_pcg_pole_reduce<1><<<a.npole, dim3(32, 8), 0, st>>>(a);
   const long nface = 2L * HALO * ((long)a.ny * a.nz + (long)a.nx * a.nz + (long)a.nx * a.ny);
   k_pcg_boundary<<<grid_blocks(nface), PT, 0, st>>>(a);
   k_pcg_fill<<<gb, PT, 0, st>>>(a);
@@ -959,8 +1243,8 @@ int pcg_issue(sb200_ctx* c, const double* d_rho, double* d_vh, int* iterations) 
   size_t nd = 0;
   SB_CUDA(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd));
   if (s->solve_grid > 0) {  // every iteration in one cooperative launch
-    const cudaError_t le = launch_solve(a, s->solve_grid, st);
-    if (le != cudaSuccess) return cuda_error(le, "k_pcg_solve (cooperative launch)");
+    const cudaError_t le = s->box.g[0] > 0 ? launch_box(a, s->box, st) : launch_solve(a, s->solve_grid, st);
+    if (le != cudaSuccess) return cuda_error(le, "CG solve (cooperative launch)");
     if (cs == cudaStreamCaptureStatusActive) return SB200_OK;
     SB_CUDA(cudaMemcpyAsync(s->host_sc, a.sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
     SB_CUDA(cudaStreamSynchronize(st));
