@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) k_collapse_batch(const BCSys* __restrict_
   collapse_item(sys[s].part, sys[s].nblk, nullptr, 0, item - first[s], sys[s].out);
 }
 
-__global__ void __launch_bounds__(256) k_finalize_batch(const FinArgs* __restrict__ args) {
+__global__ void __launch_bounds__(1024) k_finalize_batch(const FinArgs* __restrict__ args) {
   finalize_body(args[blockIdx.x]);
 }
 
@@ -500,7 +500,9 @@ int launch_obs_final_batch(sb200_batch* b, int parity, int which) {
     k_collapse_batch<<<(unsigned)((b->c_total * 32 + 255) / 256), 256, 0, b->stream>>>(b->d_csys, b->d_cfirst,
                                                                                       b->nsys);
     SB_LAUNCH_CHECK("k_collapse_batch");
-    k_finalize_batch<<<b->nsys, 256, 0, b->stream>>>(b->d_fin);
+    int nt = 0;
+    for (const sb200_ctx* s : b->sys) nt = std::max(nt, fin_threads(s->orb.norb));
+    k_finalize_batch<<<b->nsys, nt, 0, b->stream>>>(b->d_fin);
     SB_LAUNCH_CHECK("k_finalize_batch");
   }
   return SB200_OK;

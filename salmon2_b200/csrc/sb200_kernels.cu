@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(256) k_obs_sweep(const double2* __restrict__ i
       part[(long)o * a.nblk * OBS_NQ + i] = 0.0;
 }
 
-__global__ void __launch_bounds__(256) k_finalize(FinArgs a) { finalize_body(a); }
+__global__ void __launch_bounds__(1024) k_finalize(FinArgs a) { finalize_body(a); }
 
 __global__ void __launch_bounds__(256) k_collapse(const double* __restrict__ part, int nblk,
                                                   const double* __restrict__ jw, int natom, long nitems,
@@ -1377,13 +1377,13 @@ int launch_finalize(sb200_ctx* c, int itt, int nt, int trans_longi, double dt, i
     // J(t) enters calc_emfields (comm_summation over icomm_rko,
     // density_matrix.f90:448)
     a.stage = 1;
-    k_finalize<<<1, 256, 0, c->stream>>>(a);
+    k_finalize<<<1, fin_threads(a.norb), 0, c->stream>>>(a);
     SB_LAUNCH_CHECK("k_finalize");
     int r = shard_sum(c, a.sums, 7);
     if (r != SB200_OK) return r;
     a.stage = 2;
   }
-  k_finalize<<<1, 256, 0, c->stream>>>(a);
+  k_finalize<<<1, fin_threads(a.norb), 0, c->stream>>>(a);
   SB_LAUNCH_CHECK("k_finalize");
   return SB200_OK;
 }
