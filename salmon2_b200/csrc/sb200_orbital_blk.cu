@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(Blk<BZ>::BT, 1) k_step_blk(const double2* __re
   __shared__ double kn[12];
   __shared__ double red[OBS_NQ][NW];
   __shared__ double jws[NW][3];
-  __shared__ double nlred[OBS ? NW : 1][32];  // reduced nonlocal-current sums of each warp
+  __shared__ double nlred[OBS && !SPLIT ? NW : 1][32];  // reduced nonlocal-current sums of each warp
   __shared__ __align__(8) uint64_t s_bar;             // completion of the table copies
 
   const int o = blockIdx.x, t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -743,8 +743,8 @@ __global__ void __launch_bounds__(Blk<BZ>::BT, 1) k_step_blk(const double2* __re
       const int k = lane >> 2;  // rs_lane<8>(k) = 4 k
       if ((lane & 3) == 0 && k < OBS_NQ) red[k][warp] = r;
     }
-    // nonlocal current (density_matrix.f90:532-591): one warp per atom, or two
-    // per atom in the split form (their sums combined in warp order)
+    // nonlocal current (density_matrix.f90:532-591): one warp per atom, or two per
+    // atom in the split form
     double jx = 0.0, jy = 0.0, jz = 0.0;
     // chunk k of the atom's sphere (TMEM cache word i) into v: v[2c], v[2c + 1] =
     // <beta_q|psi> (c = q < 4) and <r_d beta_q|psi> (c = 4 + 3 q + d)
@@ -794,22 +794,49 @@ __global__ void __launch_bounds__(Blk<BZ>::BT, 1) k_step_blk(const double2* __re
       }
     };
     if (kb && SPLIT) {
-      const int rounds = (a.natom + NW / 2 - 1) / (NW / 2);
-      for (int rd = 0; rd < rounds; ++rd) {  // uniform over the CTA
-        const int atom = (warp >> 1) + rd * (NW / 2);
-        const int4 at = atom < a.natom ? satm[atom] : make_int4(0, 0, 0, 0);
-        double v[32];
+      // from the projections P of psi(t + dt), point by point:
+      // sum_q Im(conj(<r beta_q|psi>) P_q) = sum_j r_j Im(conj(e_j psi_j) sum_q uV_qj P_q)
+      project_half<NW>(buf, sph, suv, sap, TP, satm, ppart, a, warp, lane, kbc, tkb);
+      __syncthreads();
+      const int hf = warp & 1;
+      for (int atom = warp >> 1; atom < a.natom; atom += NW / 2) {
+        const int4 at = satm[atom];
+        if (at.w == 0) continue;
+        const double* p0 = ppart + 16 * atom;
+        double2 pq[4];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = 0.0;
-        if (at.w > 0) {
-          const int nk = (at.y + 31) >> 5;
-          for (int k = warp & 1, i = 0; k < nk; k += 2, ++i) nl_chunk(v, at.x, at.y, at.w, k, i);
+        for (int qq = 0; qq < 4; ++qq) {
+          const double rv = qq < at.w ? srinv[at.z + qq] : 0.0;
+          pq[qq] = make_double2(rv * (p0[2 * qq] + p0[8 + 2 * qq]), rv * (p0[2 * qq + 1] + p0[9 + 2 * qq]));
         }
-        const double r = warp_reduce_scatter<32>(v, lane);  // lane L holds value L
-        nlred[warp][lane] = r;
-        __syncthreads();
-        if ((warp & 1) == 0 && lane == 0 && at.w > 0) nl_atom(nlred[warp], nlred[warp + 1], at.z, at.w);
-        __syncthreads();
+        const int nk = (at.y + 31) >> 5;
+        for (int k = hf, i = 0; k < nk; k += 2, ++i) {
+          double u[4];
+          double2 e;
+          if (kbc) kb_load(tkb + 12 * i, u, e);
+          const int j = lane + 32 * k;
+          if (j >= at.y) continue;
+          const int fp = at.x + j;
+          if (!kbc) {
+#pragma unroll
+            for (int qq = 0; qq < 4; ++qq) u[qq] = suv[qq * TP + fp];
+            e = sph[fp];
+          }
+          const double2 ev = cmul(e, buf[sap[fp] & 4095]);
+          double2 sp = make_double2(0.0, 0.0);
+#pragma unroll
+          for (int qq = 0; qq < 4; ++qq) sp = make_double2(fma(u[qq], pq[qq].x, sp.x), fma(u[qq], pq[qq].y, sp.y));
+          const double im = ev.x * sp.y - ev.y * sp.x;
+          jx = fma(sr[fp], im, jx);
+          jy = fma(sr[TP + fp], im, jy);
+          jz = fma(sr[2 * TP + fp], im, jz);
+        }
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        jx += __shfl_xor_sync(0xffffffffu, jx, off);
+        jy += __shfl_xor_sync(0xffffffffu, jy, off);
+        jz += __shfl_xor_sync(0xffffffffu, jz, off);
       }
     } else if (kb) {
       for (int atom = warp; atom < a.natom; atom += NW) {
