@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256, (MODE >= 6) ? 3 : 2)
   if (nsys < 1 || nsys > MAX_SYS) return;  // the host never launches this
   unsigned char* base = tmak::tma_area(smraw);
   tmak::tma_init_barriers<MODE, false>(base);
-  uint32_t pmask = 0, amask = 0;
+  uint32_t pmask = 0, amask = 0, emask = 0;
   for (int i = threadIdx.x; i <= nsys; i += blockDim.x) sfirst[i] = first[i];
   __syncthreads();
   const long total = sfirst[nsys];
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(256, (MODE >= 6) ? 3 : 2)
     const int r = (int)(l % per_o);
     const BPtr p = ptr[s];
     const bool ok = tmak::tma_body<MODE, false>(maps[s], p.hout, p.acc, p.d32, sa, err, r % ntiles, r / ntiles, o,
-                                                base, pmask, amask);
+                                                base, pmask, amask, emask);
     __syncthreads();  // the argument block is reused by the next item
     if (!ok) break;   // a copy timed out: the flag is set, leave the queue to the others
   }

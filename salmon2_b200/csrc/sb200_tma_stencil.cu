@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(NT, (MODE >= 6) ? 3 : 2)
   extern __shared__ unsigned char smraw[];
   unsigned char* base = tma_area(smraw);
   tma_init_barriers<MODE, PER>(base);
-  uint32_t pmask = 0, amask = 0;
-  tma_body<MODE, PER>(maps, hout, acc, d32, a, err, blockIdx.x, blockIdx.y, blockIdx.z, base, pmask, amask);
+  uint32_t pmask = 0, amask = 0, emask = 0;
+  tma_body<MODE, PER>(maps, hout, acc, d32, a, err, blockIdx.x, blockIdx.y, blockIdx.z, base, pmask, amask, emask);
 }
 
 // ---------------------------------------------------------------------------
