@@ -98,13 +98,14 @@ __device__ __forceinline__ bool tile_column(int nx, int ny, int& x, int& y) {
 __device__ __forceinline__ long tile_block() { return (long)blockIdx.y * gridDim.x + blockIdx.x; }
 
 // H of real orbitals: each column marches up hz planes with the nine z neighbours
-// in registers, x and y neighbours through L1 (17 loads a point).  The KB term
-// by (point, atom) pairs from projections staged in shared memory, the point
-// map read a plane ahead: a chain of dependent loads per entry (four per pair)
-// held a warp for thousands of cycles at every plane of a sphere.  scale: null, or an
-// orbital's partial sums of <in|in> (nscale blocks): the result is that of
-// in / sqrt(<in|in>).  DOT: partial sums of <x|out> and <in scaled|out> in
-// part[o][block][2].
+// in registers; x and y neighbours from the plane's tile with its 4-point halo
+// (zero outside an isolated grid) in shared memory, the next plane's loads
+// issued before this one's sums.  (Neighbours through L1 took a test, a select
+// and an address each: 200 instructions a point and plane, 45 of them FP64.)
+// The KB term by (point, atom) pairs from projections staged in shared memory,
+// the point map read a plane ahead.  scale: null, or an orbital's partial sums
+// of <in|in> (nscale blocks): the result is that of in / sqrt(<in|in>).  DOT:
+// partial sums of <x|out> and <in scaled|out> in part[o][block][2].
 constexpr int HMAX_NLMA = 1024;
 template <bool DOT>
 __global__ void __launch_bounds__(HX* HY) k_dhpsi(const double* __restrict__ in, double* __restrict__ out, RArgs a,
@@ -129,50 +130,65 @@ __global__ void __launch_bounds__(HX* HY) k_dhpsi(const double* __restrict__ in,
   }
   __syncthreads();
   double d[2] = {0.0, 0.0};
-  if (act) {
-    const double* src = in + (long)o * a.npts;
-    const int plane = a.nx * a.ny, col = x + a.nx * y;
-    int xo[2 * ND], yo[2 * ND];
-    unsigned ok = 0;  // bit per x / y neighbour: inside the grid
+  const double* src = in + (long)o * a.npts;
+  const int plane = a.nx * a.ny, col = act ? x + a.nx * y : 0;
+  constexpr int SX = HX + 2 * ND, NS = SX * (HY + 2 * ND), SL = (NS + HX * HY - 1) / (HX * HY);
+  __shared__ double tile[2][NS];
+  const int x0 = x - (int)(threadIdx.x % HX), y0 = y - (int)(threadIdx.x / HX);
+  int goff[SL];  // plane offset of the tile values this thread loads, -1: zero
 #pragma unroll
-    for (int s = 1; s <= ND; ++s) {
-      bool b0, b1, b2, b3;
-      xo[2 * s - 2] = wrap(x + s, a.nx, a.periodic, b0) - x;
-      xo[2 * s - 1] = wrap(x - s, a.nx, a.periodic, b1) - x;
-      yo[2 * s - 2] = (wrap(y + s, a.ny, a.periodic, b2) - y) * a.nx;
-      yo[2 * s - 1] = (wrap(y - s, a.ny, a.periodic, b3) - y) * a.nx;
-      ok |= ((unsigned)b0 | (unsigned)b1 << 1 | (unsigned)b2 << 2 | (unsigned)b3 << 3) << (4 * (s - 1));
+  for (int i = 0; i < SL; ++i) {
+    const int e = threadIdx.x + i * HX * HY;
+    int gx = x0 - ND + e % SX, gy = y0 - ND + e / SX;
+    goff[i] = -1;
+    if (e >= NS) continue;
+    if (a.periodic) {
+      gx = gx % a.nx;
+      gy = gy % a.ny;
+      gx = gx < 0 ? gx + a.nx : gx;
+      gy = gy < 0 ? gy + a.ny : gy;
     }
-    auto ldz = [&](int z) -> double {
-      bool in_grid;
-      const int q = wrap(z, a.nz, a.periodic, in_grid);
-      return in_grid ? __ldg(src + (long)q * plane + col) : 0.0;
-    };
-    const int* map = a.pairs ? a.pmap2 : a.pmap;
-    double w[2 * ND + 1];
+    if (gx >= 0 && gx < a.nx && gy >= 0 && gy < a.ny) goff[i] = gx + a.nx * gy;
+  }
+  auto ldz = [&](int z) -> double {
+    bool in_grid;
+    const int q = wrap(z, a.nz, a.periodic, in_grid);
+    return in_grid && act ? __ldg(src + (long)q * plane + col) : 0.0;
+  };
+  const int* map = a.pairs ? a.pmap2 : a.pmap;
+  double w[2 * ND + 1], v[SL];
 #pragma unroll
-    for (int i = 0; i < 2 * ND; ++i) w[i] = ldz(z0 - ND + i);
-    const double* V = a.vloc + (long)(o % a.nspin) * a.npts;
-    int pn = a.nlma > 0 ? __ldg(map + (long)z0 * plane + col) : -1;
-    for (int z = z0; z < z1; ++z) {
-      w[2 * ND] = ldz(z + ND);
-      const long p = (long)z * plane + col;
-      const double* P = src + p;
-      const int pm = pn;
-      if (a.nlma > 0 && z + 1 < z1) pn = __ldg(map + p + plane);
+  for (int i = 0; i < 2 * ND; ++i) w[i] = ldz(z0 - ND + i);
+#pragma unroll
+  for (int i = 0; i < SL; ++i) v[i] = goff[i] >= 0 ? __ldg(src + (long)z0 * plane + goff[i]) : 0.0;
+  const double* V = a.vloc + (long)(o % a.nspin) * a.npts;
+  int pn = a.nlma > 0 && act ? __ldg(map + (long)z0 * plane + col) : -1;
+  const int ctr = (threadIdx.x / HX + ND) * SX + threadIdx.x % HX + ND;
+  for (int z = z0; z < z1; ++z) {
+    double* T = tile[z & 1];
+#pragma unroll
+    for (int i = 0; i < SL; ++i)
+      if (threadIdx.x + i * HX * HY < NS) T[threadIdx.x + i * HX * HY] = v[i];
+    __syncthreads();
+    w[2 * ND] = ldz(z + ND);
+    const int p = z * plane + col;
+    const int pm = pn;
+    if (z + 1 < z1) {
+      if (a.nlma > 0 && act) pn = __ldg(map + p + plane);
+#pragma unroll
+      for (int i = 0; i < SL; ++i) v[i] = goff[i] >= 0 ? __ldg(src + (long)(z + 1) * plane + goff[i]) : 0.0;
+    }
+    if (act) {
+      const double vl = __ldg(V + p);
       double vx = 0.0, vy = 0.0, vz = 0.0;
 #pragma unroll
       for (int s = 0; s < ND; ++s) {
-        const double xp = (ok >> (4 * s)) & 1 ? __ldg(P + xo[2 * s]) : 0.0;
-        const double xm = (ok >> (4 * s + 1)) & 1 ? __ldg(P + xo[2 * s + 1]) : 0.0;
-        const double yp = (ok >> (4 * s + 2)) & 1 ? __ldg(P + yo[2 * s]) : 0.0;
-        const double ym = (ok >> (4 * s + 3)) & 1 ? __ldg(P + yo[2 * s + 1]) : 0.0;
-        vx += a.lapt[s] * (xp + xm);
-        vy += a.lapt[ND + s] * (yp + ym);
+        vx += a.lapt[s] * (T[ctr + s + 1] + T[ctr - s - 1]);
+        vy += a.lapt[ND + s] * (T[ctr + (s + 1) * SX] + T[ctr - (s + 1) * SX]);
         vz += a.lapt[2 * ND + s] * (w[ND + 1 + s] + w[ND - 1 - s]);
       }
       const double c = w[ND];
-      double h = (__ldg(V + p) + a.lap0) * c - 0.5 * (vz + (vy + vx));
+      double h = (vl + a.lap0) * c - 0.5 * (vz + (vy + vx));
       if (pm >= 0) {
         const int e1 = (pm >> 8) + (pm & 255);
         if (a.pairs) {
@@ -196,9 +212,9 @@ __global__ void __launch_bounds__(HX* HY) k_dhpsi(const double* __restrict__ in,
         d[0] = fma(__ldg(xk + (long)o * a.npts + p), h, d[0]);
         d[1] = fma(f * c, h, d[1]);
       }
-#pragma unroll
-      for (int i = 0; i < 2 * ND; ++i) w[i] = w[i + 1];
     }
+#pragma unroll
+    for (int i = 0; i < 2 * ND; ++i) w[i] = w[i + 1];
   }
   if (DOT) {
     block_totals<2, HX * HY>(d, red);
