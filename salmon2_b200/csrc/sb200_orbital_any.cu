@@ -15,13 +15,19 @@
 //
 // Per term: partial Kleinman-Bylander projections of the slab's sphere points
 // (warps per atom; each atom's points are sorted by grid point, so a slab's
-// part is one run) and the stencil sweep; cluster barrier; every CTA adds the C partial sums in rank order, forms the
-// contribution of each of its (point, atom) pairs, and the owners finish h_n = stencil + pairs, update
+// part is one run) and the stencil sweep; cluster barrier; every CTA adds the C
+// partial sums (a lane to each rank's), forms the contribution of each of its
+// (point, atom) pairs, and the owners finish h_n = stencil + pairs, update
 // psi_out and overwrite h_{n-1}; cluster barrier.  After the last term the
 // observables of psi(t+dt), added over the cluster in rank order by CTA 0; its
 // nonlocal current from the projections P of psi(t+dt), pair by pair:
 // sum_j r_j Im(conj(e_j psi_j) sum_q uV_qj P_q), which is the sum over q of
 // Im(conj(<r beta_q|psi>) P_q).  HBM: psi in, psi_out out.
+//
+// The KB tables are read twice a term, from L2 where they are large; STAGE keeps
+// the slab's in shared memory (60 bytes a pair) where they fit beside the
+// orbital: small cells, where a term is a chain of latencies (12^3 x 32 orbitals,
+// a step with its observables: 41.5 -> 33 us).
 //
 // Bound inside the SM: per point and term 96 FP64 operations of the stencil
 // (64 lanes a cycle) against 18 shared-memory loads of 16 bytes (128 bytes a
@@ -52,7 +58,6 @@ namespace {
 
 constexpr int MAX_NT = 512;
 constexpr int MAX_NW = MAX_NT / 32;
-constexpr int U = 3;  // plane steps unrolled
 
 struct AnyArgs {
   int nx, ny, nz, ncol;  // ncol = nx ny columns
@@ -69,6 +74,7 @@ struct AnyArgs {
   const int* pst;        // [natom][nz + 1] first flat sphere point of the atom at or above each plane
   const int* ppl;        // [nz + 1] first (point, atom) pair at or above each plane
   const int* pt_lin;
+  const int* apj;        // [totpts] pair of each sphere point
   const double* uv4;     // [totpts][4]
   const double* pt_r;    // [totpts][3]
   const double2* phase;  // [nk][totpts]
@@ -86,7 +92,8 @@ struct AnyArgs {
   double* jw;              // [norb][3] or null
   int* err;
   // byte offsets into dynamic shared memory (after the slab)
-  unsigned o_pc, o_part, o_proj, o_atom, o_ptab, o_rinv, o_pm;
+  unsigned o_pc, o_part, o_proj, o_atom, o_ptab, o_rinv, o_pm, o_tab, o_idx;
+  int maxpairs;            // most pairs of a slab
 };
 constexpr int NB = 4;     // sphere points, pairs or grid points of a thread in flight at once
 constexpr int NSUM = 10;  // sums of an orbital: OBS_NQ and the nonlocal current
@@ -144,7 +151,8 @@ __device__ __forceinline__ void unrolled(F& f, int k0, int n) {
   }
 }
 
-template <bool OBS>
+// STAGE: the slab's KB tables stay in shared memory for the whole step
+template <bool OBS, bool STAGE>
 __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restrict__ in, double2* __restrict__ out,
                                                         const __grid_constant__ AnyArgs a,
                                                         const __grid_constant__ StepZC zc, int nterm) {
@@ -157,6 +165,14 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
   const double2** ptab = (const double2**)(sraw + a.o_ptab);  // [nz] plane pointers, own and the neighbours'
   double* srinv = (double*)(sraw + a.o_rinv);      // [nlma]
   int* spm = (int*)(sraw + a.o_pm);                // [D][ncol] point map of the slab
+  // STAGE: per pair of the slab the phase and the four uV (three runs of 16 bytes)
+  // and first ilma | projectors << 24; per sphere point its pair and its point
+  double2* te = (double2*)(sraw + a.o_tab);
+  double2* tu0 = te + a.maxpairs;
+  double2* tu1 = tu0 + a.maxpairs;
+  int* tlm = (int*)(tu1 + a.maxpairs);
+  int2* tix = (int2*)(sraw + a.o_idx);
+  int* sbase = (int*)ppart;  // (before the first projections)
   __shared__ uint32_t s_tmem;
   __shared__ __align__(16) double kn[12];
   __shared__ double red[NSUM][MAX_NW];
@@ -189,7 +205,8 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
   if (kb) {
     for (int i = t; i < a.natom; i += NT) {
       const int* ps = a.pst + (long)i * (a.nz + 1);
-      satm[i] = make_int4(__ldg(ps + z0), __ldg(ps + z0 + D), __ldg(a.lma_start + i), __ldg(a.nproj + i));
+      const int np = __ldg(a.nproj + i), j0 = __ldg(ps + z0);  // (no projectors: no pairs, an empty run)
+      satm[i] = make_int4(j0, np > 0 ? __ldg(ps + z0 + D) : j0, __ldg(a.lma_start + i), np);
     }
     for (int i = t; i < a.nlma; i += NT) srinv[i] = __ldg(a.rinv + i);
 #pragma unroll 8
@@ -206,6 +223,31 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
   tmem::fence_after_sync();
   const uint32_t tb = tmem::warp_addr(s_tmem, warp, (uint32_t)(warp >> 2) * (uint32_t)a.tw);
   const int pb0 = kb ? __ldg(a.ppl + z0) : 0, pb1 = kb ? __ldg(a.ppl + z0 + D) : 0;
+  if (STAGE && kb) {
+    for (int i = t; i < pb1 - pb0; i += NT) {
+      const int pr = pb0 + i;
+      te[i] = __ldg(a.pair_ph + (long)ik * a.npair + pr);
+      tu0[i] = __ldg((const double2*)a.pair_uv + 2 * pr);
+      tu1[i] = __ldg((const double2*)a.pair_uv + 2 * pr + 1);
+      tlm[i] = __ldg(a.pair_lma + pr);
+    }
+    // the runs of the atoms one after the other; satm then counts in tix
+    for (int atom = warp; atom < a.natom; atom += NW) {
+      int n = 0;
+      for (int i = lane; i < atom; i += 32) n += satm[i].y - satm[i].x;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
+      const int4 at = satm[atom];
+      for (int j = at.x + lane; j < at.y; j += 32)
+        tix[n + j - at.x] = make_int2(__ldg(a.apj + j) - pb0, __ldg(a.pt_lin + j) - z0 * ncol);
+      if (lane == 0) sbase[atom] = n;
+    }
+    __syncthreads();
+    for (int i = t; i < a.natom; i += NT) {
+      const int4 at = satm[i];
+      satm[i] = make_int4(sbase[i], sbase[i] + at.y - at.x, at.z, at.w);
+    }
+  }
   const double2* ph = kb ? a.phase + (long)ik * a.totpts : nullptr;
   const double2* pph = kb ? a.pair_ph + (long)ik * a.npair : nullptr;
   if (!tma::mbar_wait(&s_bar, 0)) {  // bounded; the step goes on to its barriers with the flag set
@@ -232,9 +274,16 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
           const int j = min(j0 + i * 32 * a.npart, at.y - 1);
-          ev[i] = cmul(__ldg(ph + j), buf[__ldg(a.pt_lin + j) - z0 * ncol]);
-          u0[i] = __ldg((const double2*)a.uv4 + 2 * j);
-          u1[i] = __ldg((const double2*)a.uv4 + 2 * j + 1);
+          if (STAGE) {
+            const int2 x = tix[j];
+            ev[i] = cmul(te[x.x], buf[x.y]);
+            u0[i] = tu0[x.x];
+            u1[i] = tu1[x.x];
+          } else {
+            ev[i] = cmul(__ldg(ph + j), buf[__ldg(a.pt_lin + j) - z0 * ncol]);
+            u0[i] = __ldg((const double2*)a.uv4 + 2 * j);
+            u1[i] = __ldg((const double2*)a.uv4 + 2 * j + 1);
+          }
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
@@ -255,19 +304,24 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
   };
   // the projections from the cluster's partial sums (after a cluster barrier)
   auto gather = [&]() {
-    for (int i = t; i < 4 * a.natom; i += NT) {
-      const int atom = i >> 2, q = i & 3;
-      const int4 at = satm[atom];
-      if (q < at.w) {
-        double2 s = make_double2(0.0, 0.0);
-#pragma unroll 4
-        for (int r = 0; r < C; ++r) {
-          const double* pr = C > 1 ? cl.map_shared_rank(ppart, r) : ppart;
-          for (int p = 0; p < a.npart; ++p) {
-            const double2 v = *(const double2*)(pr + 8 * (atom * a.npart + p) + 2 * q);
-            s = make_double2(s.x + v.x, s.y + v.y);
-          }
+    // C lanes to a projection, one per rank: the remote loads of all in flight at
+    // once; added by butterfly over the ranks
+    const int items = 4 * a.natom * C, r = t & (C - 1);
+    const double* pr = C > 1 ? cl.map_shared_rank(ppart, r) : ppart;
+    for (int i0 = warp * 32; i0 < items; i0 += NT) {
+      const int i = (i0 + lane) / C, atom = i >> 2, q = i & 3;
+      const int4 at = i0 + lane < items ? satm[atom] : make_int4(0, 0, 0, 0);
+      double2 s = make_double2(0.0, 0.0);
+      if (q < at.w)
+        for (int p = 0; p < a.npart; ++p) {
+          const double2 v = *(const double2*)(pr + 8 * (atom * a.npart + p) + 2 * q);
+          s = make_double2(s.x + v.x, s.y + v.y);
         }
+      for (int off = 1; off < C; off <<= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, off);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, off);
+      }
+      if (r == 0 && q < at.w) {
         const double rv = srinv[at.z + q];
         sproj[at.z + q] = make_double2(rv * s.x, rv * s.y);
       }
@@ -279,6 +333,13 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
     double2 e, u0, u1;
   };
   auto load_pair = [&](Pair& f, int pr) {
+    if (STAGE) {
+      f.lm = tlm[pr - pb0];
+      f.e = te[pr - pb0];
+      f.u0 = tu0[pr - pb0];
+      f.u1 = tu1[pr - pb0];
+      return;
+    }
     f.lm = __ldg(a.pair_lma + pr);
     f.e = __ldg(pph + pr);
     f.u0 = __ldg((const double2*)a.pair_uv + 2 * pr);
@@ -309,7 +370,7 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
           xo[s - 1] = (xp & 0xffff) | (int)((unsigned)xm << 16);
           yo[s - 1] = (yp & 0xffff) | (int)((unsigned)ym << 16);
         }
-        double2 w[2 * ND + U];  // step j of a group of U reads w[j .. j + 8]
+        double2 w[2 * ND + 1];  // rolls through registers (steps unrolled by 3 or 9 cost more in fetches: 35, 40 : 33 us)
 #pragma unroll
         for (int i = 0; i < 2 * ND; ++i) {
           int z = z0 - ND + i;
@@ -317,13 +378,13 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
           w[i] = ptab[z][c];
         }
         double dn = __ldg(vsl + c);
-        auto step = [&](auto jc, const int k) {
-          constexpr int j = decltype(jc)::value;
+#pragma unroll 1
+        for (int k = 0; k < D; ++k) {
           int z = z0 + k + ND;
           z = z >= a.nz ? z - a.nz : z;
-          w[j + 2 * ND] = ptab[z][c];
+          w[2 * ND] = ptab[z][c];
           const double2* P = buf + k * ncol + c;
-          const double2 cv = w[j + ND];
+          const double2 cv = w[ND];
           const double dg = dn + lap0;
           dn = __ldg(vsl + min(k + 1, D - 1) * ncol + c);
           // one accumulator per axis: chains of 8 dependent FMA instead of 24
@@ -334,10 +395,10 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
             const double2 kz = *(const double2*)(kn + 8 + s);
             pair_acc(hx, P[(short)xo[s]], P[xo[s] >> 16], a.mhl[s], kx.x);
             pair_acc(hy, P[(short)yo[s]], P[yo[s] >> 16], a.mhl[4 + s], ky.x);
-            pair_acc(hz, w[j + ND + 1 + s], w[j + ND - 1 - s], a.mhl[8 + s], kz.x);
+            pair_acc(hz, w[ND + 1 + s], w[ND - 1 - s], a.mhl[8 + s], kz.x);
             pair_acc(hx, P[(short)xo[s + 1]], P[xo[s + 1] >> 16], a.mhl[s + 1], kx.y);
             pair_acc(hy, P[(short)yo[s + 1]], P[yo[s + 1] >> 16], a.mhl[5 + s], ky.y);
-            pair_acc(hz, w[j + ND + 2 + s], w[j + ND - 2 - s], a.mhl[9 + s], kz.y);
+            pair_acc(hz, w[ND + 2 + s], w[ND - 2 - s], a.mhl[9 + s], kz.y);
           }
           const double2 h = make_double2((hx.x + hy.x) + hz.x, (hx.y + hy.y) + hz.y);
           const uint32_t ta = tb + 8 * (rd * a.dmax + k);
@@ -349,11 +410,8 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
             const uint32_t hw[4] = {tmem::lo_word(h.x), tmem::hi_word(h.x), tmem::lo_word(h.y), tmem::hi_word(h.y)};
             tmem::st4_async(ta, hw);
           }
-        };
-        for (int k0 = 0; k0 < D; k0 += U) {
-          unrolled<0, U>(step, k0, D);
 #pragma unroll
-          for (int i = 0; i < 2 * ND; ++i) w[i] = w[i + U];
+          for (int i = 0; i < 2 * ND; ++i) w[i] = w[i + 1];
         }
       }
     };
@@ -528,11 +586,13 @@ __global__ void __launch_bounds__(MAX_NT, 1) k_step_any(const double2* __restric
 // Shape of the launch with clusters of C CTAs: false when the orbital does not fit.
 struct AnyShape {
   int C = 0, NT = 0, rounds = 0, dmax = 0, tw = 0, npart = 1;
-  unsigned tcols = 0, o_pc = 0, o_part = 0, o_proj = 0, o_atom = 0, o_ptab = 0, o_rinv = 0, o_pm = 0;
+  bool stage = false;
+  int maxpairs = 0;
+  unsigned tcols = 0, o_tab = 0, o_idx = 0, o_pc = 0, o_part = 0, o_proj = 0, o_atom = 0, o_ptab = 0, o_rinv = 0, o_pm = 0;
   size_t smem = 0;
 };
 
-bool any_shape(const sb200_ctx* c, int C, AnyShape* s) {
+bool any_shape(const sb200_ctx* c, int C, bool stage, AnyShape* s) {
   const GridInfo& g = c->g;
   const PPInfo& pp = c->pp;
   if (C > g.nz) return false;
@@ -569,6 +629,14 @@ bool any_shape(const sb200_ctx* c, int C, AnyShape* s) {
   off += up((size_t)(kb ? pp.nlma : 0) * 8);
   s->o_pm = (unsigned)off;
   off += up(kb ? (size_t)s->dmax * ncol * 4 : 0);
+  s->stage = stage && kb;
+  s->maxpairs = (int)pairs;
+  if (s->stage) {  // pairs and sphere points are one to one
+    s->o_tab = (unsigned)off;
+    off += up(pairs * 52);
+    s->o_idx = (unsigned)off;
+    off += up(pairs * 8);
+  }
   // CTAs that share an SM share its 512 TMEM columns: each takes at least the
   // same share of its 228 KB of shared memory (1 KB of it the system's, some
   // static), so that an allocation never waits for another CTA's columns
@@ -596,7 +664,7 @@ cudaLaunchConfig_t any_config(const AnyShape& s, int norb, cudaStream_t st, cuda
 void any_limits(sb200_ctx* c) {
   static const int stat = [] {
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, k_step_any<true>) != cudaSuccess) {
+    if (cudaFuncGetAttributes(&fa, k_step_any<true, false>) != cudaSuccess) {
       cudaGetLastError();
       return -1;
     }
@@ -604,8 +672,10 @@ void any_limits(sb200_ctx* c) {
   }();
   int optin = 0;
   if (stat < 0 || cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess ||
-      cudaFuncSetAttribute(k_step_any<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - stat) != cudaSuccess ||
-      cudaFuncSetAttribute(k_step_any<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - stat) != cudaSuccess) {
+      cudaFuncSetAttribute(k_step_any<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - stat) != cudaSuccess ||
+      cudaFuncSetAttribute(k_step_any<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - stat) != cudaSuccess ||
+      cudaFuncSetAttribute(k_step_any<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - stat) != cudaSuccess ||
+      cudaFuncSetAttribute(k_step_any<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - stat) != cudaSuccess) {
     cudaGetLastError();
     c->any_smem_cap = 0;
     return;
@@ -630,8 +700,9 @@ void any_plan(sb200_ctx* c) {
   double best = 0.0;
   for (int C = 1; C <= 8; C *= 2) {
     AnyShape s;
-    if (!any_shape(c, C, &s)) continue;
     if (force && atoi(force) != C) continue;
+    // with the tables in shared memory where they fit
+    if (!any_shape(c, C, true, &s) && !any_shape(c, C, false, &s)) continue;
     // CTAs an SM holds (shared memory, registers, threads), and the clusters at
     // work at a time: clusters stay within a GPC, which leaves some SMs out
     // (35 clusters of 4 and 17 of 8 were seen with one CTA per SM)
@@ -640,13 +711,17 @@ void any_plan(sb200_ctx* c) {
     if (per_sm < 1) continue;
     const int nclus = (C == 1 ? 148 : 140) * per_sm / C;
     // cycles of a term, from stamps of the phases on 12^3, 21 x 18 x 15 and 32^3
-    // cells: barriers; the sweep's 8 + D planes a column, each bound by its own
-    // chain of loads (700 cycles) or by the shared-memory loads of the warps on
-    // the SM (70 each); three cycles a point for the rest.  Times the waves.
+    // cells: barriers; the sweep's planes a column, D of its own and eight of the
+    // neighbours', each bound by its own chain of loads (700 cycles) or by the
+    // shared-memory loads of the warps on the SM (70 each), the neighbours' also
+    // by the other CTAs' remote loads; three cycles a point for the rest.  Times
+    // the waves.  (12^3, 32 orbitals: 55, 43, 35 and 43 us with 1, 2, 4 and 8 CTAs;
+    // 21 x 18 x 15, 270 orbitals: 174, 235, 373 and 628.)
     const double waves = (double)((c->orb.norb + nclus - 1) / nclus);
     const double share = std::max(1.0, std::min((double)c->orb.norb, (double)nclus) * C / 148.0);  // CTAs per SM
-    const double plane = std::max(700.0, 70.0 * (s.NT / 32) * share);
-    const double cost = waves * (3000.0 + (C > 1 ? 6000.0 : 0.0) + s.rounds * (s.dmax + 8) * plane +
+    const double lds = 70.0 * (s.NT / 32);
+    const double own = std::max(700.0, lds * share), other = (C > 1 ? share : 1.0) * std::max(700.0, lds);
+    const double cost = waves * (3000.0 + (C > 1 ? 2000.0 : 0.0) + s.rounds * (s.dmax * own + 8 * other) +
                                  3.0 * s.dmax * g.nx * g.ny * share);
     if (c->any_C == 0 || cost < best) {
       best = cost;
@@ -670,7 +745,8 @@ bool step_any_applies(sb200_ctx* c, int n_hamil) {
 int launch_step_any(sb200_ctx* c, const double2* in, double2* out, const double2* zc, int n_hamil, bool with_obs,
                     bool hmode) {
   AnyShape s;
-  if (!any_shape(c, c->any_C, &s)) return set_error(SB200_ERR_BAD_SHAPE, "fused step: the orbital does not fit");
+  if (!any_shape(c, c->any_C, true, &s) && !any_shape(c, c->any_C, false, &s))
+    return set_error(SB200_ERR_BAD_SHAPE, "fused step: the orbital does not fit");
   const GridInfo& g = c->g;
   const PPInfo& pp = c->pp;
   AnyArgs a;
@@ -719,6 +795,10 @@ int launch_step_any(sb200_ctx* c, const double2* in, double2* out, const double2
   a.o_proj = s.o_proj;
   a.o_atom = s.o_atom;
   a.o_ptab = s.o_ptab;
+  a.o_tab = s.o_tab;
+  a.o_idx = s.o_idx;
+  a.maxpairs = s.maxpairs;
+  a.apj = pp.d_apj;
   a.o_rinv = s.o_rinv;
   a.o_pm = s.o_pm;
   a.pair_pt = pp.d_pair_pt;
@@ -728,8 +808,10 @@ int launch_step_any(sb200_ctx* c, const double2* in, double2* out, const double2
   for (int i = 0; i < STEP_MAX_NTERM; ++i) z.v[i] = (zc && i < n_hamil) ? zc[i] : make_double2(0.0, 0.0);
   cudaLaunchAttribute at;
   const cudaLaunchConfig_t cfg = any_config(s, c->orb.norb, c->stream, &at);
-  if (with_obs) SB_CUDA(cudaLaunchKernelEx(&cfg, k_step_any<true>, in, out, a, z, n_hamil));
-  else SB_CUDA(cudaLaunchKernelEx(&cfg, k_step_any<false>, in, out, a, z, n_hamil));
+  void (*fn)(const double2*, double2*, AnyArgs, StepZC, int) =
+      with_obs ? (s.stage ? k_step_any<true, true> : k_step_any<true, false>)
+               : (s.stage ? k_step_any<false, true> : k_step_any<false, false>);
+  SB_CUDA(cudaLaunchKernelEx(&cfg, fn, in, out, a, z, n_hamil));
   return SB200_OK;
 }
 
