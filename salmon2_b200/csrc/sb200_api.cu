@@ -79,7 +79,8 @@ int ensure_stage(sb200_ctx* c, size_t bytes) {
 
 // (re)allocate work buffers that depend on grid x orbitals x projectors
 int ensure_work(sb200_ctx* c) {
-  c->any_C = -1;  // the fused step's shape is chosen anew
+  c->any_C = -1;  // the shapes of the fused step and the non-orthogonal sweep are chosen anew
+  c->no_tile = {};
   if (!c->g.set || !c->orb.set) return SB200_OK;
   dfree(c->d_proj);
   dfree(c->d_jw);
@@ -482,7 +483,6 @@ int sb200_ctx_destroy(sb200_ctx* c) {
   learned_free(c);
   scf_free(c);
   pcg_free(c);
-  dfree(c->d_nonorth);
   dfree(c->d_acm);
   dfree(c->d_divac);
   dfree(c->d_mcur);
@@ -915,10 +915,7 @@ int sb200_set_lattice(sb200_ctx* c, const double rmatrix_B[9], const double coef
     for (int i = 0; i < 6; ++i) c->g.coefF[i] = coef_F[i];
     c->g.nonorth = 1;
   }
-  if (c->orb.set) {
-    TRY(refresh_k(c));
-    TRY(nonorth_prepare(c));  // the two-pass scratch at set-up, not inside a later capture
-  }
+  if (c->orb.set) TRY(refresh_k(c));
   return SB200_OK;
 }
 
@@ -1267,7 +1264,6 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
   double2* B = (double2*)psi_b;
   double2* W = (double2*)work;
   TRY(scf_rt_prepare(c));
-  TRY(nonorth_prepare(c));
   if (c->length_gauge && !c->g.periodic) {  // E_ext(itt) = -(Ac_ext(itt+1) - Ac_ext(itt)) / dt, initialization_rt.f90:180-183
     std::vector<double> ac(na, 0.0), e(na, 0.0);
     if (Ac_ext) SB_CUDA(cudaMemcpy(ac.data(), Ac_ext, na * sizeof(double), cudaMemcpyDefault));

@@ -141,6 +141,12 @@ struct GSState {
 
 }  // namespace sb200
 
+// Column tile, threads and z chunks of the non-orthogonal sweep; w = 0: not chosen yet.
+struct NonorthTile {
+  int w = 0, h = 0, NT = 0, nchunk = 1;
+  size_t smem = 0;
+};
+
 struct sb200_ctx {
   int device = 0;
   cudaStream_t own_stream = nullptr;
@@ -172,6 +178,7 @@ struct sb200_ctx {
   void* d_stage = nullptr;      // relayout staging
   size_t stage_bytes = 0;
   bool vloc_set = false;
+  NonorthTile no_tile;
   int any_C = -1;              // cluster size of the fused step of general periodic grids (0: does not apply,
                                // -1: to be chosen at the next step)
   int any_resident = 0;        // its clusters at work at a time
@@ -203,9 +210,6 @@ struct sb200_ctx {
   void* scf = nullptr;
   // isolated Hartree potential by CG (sb200_poisson_cg.cu)
   void* pcg = nullptr;
-  // non-orthogonal H psi: first-pass H psi and the x / y first derivatives [3][norb][npts]
-  double2* d_nonorth = nullptr;
-  size_t nonorth_cap = 0;
   // single-scale Maxwell-TDDFT (sb200_set_micro_ac): Ac_micro [npts][3] and div Ac [npts]
   int microac = 0;
   int micro_sym = 0;  // sb200_set_symmetrized_stencil
@@ -300,7 +304,7 @@ int launch_project_dmma(sb200_ctx* c, const void* in, double2* proj, bool in32);
 // 2 n^2 doubles; *info = 1 when the QL iterations did not converge (sb200_eigh.cu)
 int launch_eigh(sb200_ctx* c, const double* M, int n, double* work, double* V, double* w, int* info);
 int launch_hpsi(sb200_ctx* c, const HpsiLaunch& L);
-int nonorth_prepare(sb200_ctx* c);  // scratch of the non-orthogonal hpsi, before a graph capture
+int launch_hpsi_nonorth(sb200_ctx* c, const HpsiLaunch& L);  // sb200_nonorth.cu
 int launch_hpsi_tiled(sb200_ctx* c, const HpsiLaunch& L);  // sb200_stencil.cu
 // tensor-copy-fed tiled kernel; SB200_ERR_UNSUPPORTED when it does not apply (sb200_tma_stencil.cu)
 int launch_hpsi_tma(sb200_ctx* c, const HpsiLaunch& L);

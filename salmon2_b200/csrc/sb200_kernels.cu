@@ -747,145 +747,10 @@ int launch_energy_parts(sb200_ctx* c, const double2* psi, const double2* h, cons
   return SB200_OK;
 }
 
-// ---------------------------------------------------------------------------
-// hpsi on a non-orthogonal lattice (zstencil_nonorthogonal, stencil.f90:120-214,
-// called from hamiltonian.f90:306-357), one thread per point in two passes:
-// (1) the lattice-axis sums v_d = sum_s lapt(s,d) (t+ + t-) and the first
-// derivatives w_d = sum_s nab(s,d) (t+ - t-), h = (V + k_lap0) psi
-// - 1/2 sum F_d v_d - i sum Bk_d w_d with Bk = B (k+A); w_x and w_y stored;
-// (2) the mixed terms - 1/2 (F_4 d_z w_y + F_5 d_z w_x + F_6 d_y w_x) from the
-// stored derivatives, then the KB term through the inverse map and the Taylor
-// epilogue of MODE.  Periodic grids only (the neighbours wrap).
-// ---------------------------------------------------------------------------
+// first-derivative coefficients of the single-scale kernels
 struct NoArgs {
-  double F[6], nab[12];
+  double nab[12];
 };
-
-__device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
-
-__global__ void __launch_bounds__(256) k_hpsi_no1(const double2* __restrict__ in, double2* __restrict__ h1,
-                                                  double2* __restrict__ wx, double2* __restrict__ wy, HArgs a,
-                                                  NoArgs n) {
-  const long p = blockIdx.x * 256L + threadIdx.x;
-  if (p >= a.npts) return;
-  const int o = blockIdx.y;
-  const int x = (int)(p % a.nx), y = (int)((p / a.nx) % a.ny), z = (int)(p / ((long)a.nx * a.ny));
-  const double2* src = in + (long)o * a.npts;
-  const int ik = o / a.nspin_no, ispin = o % a.nspin;
-  const double* kc = a.kcoef + (long)KC * ik;
-  const long sy = a.nx, sz = (long)a.nx * a.ny;
-  double2 v[3], w[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double2 vv = make_double2(0.0, 0.0), ww = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int s = 1; s <= ND; ++s) {
-      long qp, qm;
-      if (d == 0) {
-        qp = p - x + wrapi(x + s, a.nx);
-        qm = p - x + wrapi(x - s, a.nx);
-      } else if (d == 1) {
-        qp = p + (long)(wrapi(y + s, a.ny) - y) * sy;
-        qm = p + (long)(wrapi(y - s, a.ny) - y) * sy;
-      } else {
-        qp = p + (long)(wrapi(z + s, a.nz) - z) * sz;
-        qm = p + (long)(wrapi(z - s, a.nz) - z) * sz;
-      }
-      const double2 tp = __ldg(src + qp), tm = __ldg(src + qm);
-      vv = cadd(vv, cscal(a.lapt[4 * d + s - 1], cadd(tp, tm)));
-      ww = cadd(ww, cscal(n.nab[4 * d + s - 1], csub(tp, tm)));
-    }
-    v[d] = vv;
-    w[d] = ww;
-  }
-  const double2 c = __ldg(src + p);
-  const double dg = __ldg(a.vloc + (long)ispin * a.npts + p) + kc[3];
-  const double2 fv = cadd(cadd(cscal(n.F[0], v[0]), cscal(n.F[1], v[1])), cscal(n.F[2], v[2]));
-  const double2 bw = cadd(cadd(cscal(kc[16], w[0]), cscal(kc[17], w[1])), cscal(kc[18], w[2]));
-  // (V + lap0) psi - 0.5 (F.v) - i (Bk.w)
-  const long gi = (long)o * a.npts + p;
-  h1[gi] = make_double2(dg * c.x - 0.5 * fv.x + bw.y, dg * c.y - 0.5 * fv.y - bw.x);
-  wx[gi] = w[0];
-  wy[gi] = w[1];
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(256) k_hpsi_no2(const double2* __restrict__ in, const double2* __restrict__ h1,
-                                                  const double2* __restrict__ wx, const double2* __restrict__ wy,
-                                                  double2* __restrict__ hout, double2* __restrict__ acc, HArgs a,
-                                                  NoArgs n) {
-  const long p = blockIdx.x * 256L + threadIdx.x;
-  if (p >= a.npts) return;
-  const int o = blockIdx.y;
-  const int y = (int)((p / a.nx) % a.ny), z = (int)(p / ((long)a.nx * a.ny));
-  const long sy = a.nx, sz = (long)a.nx * a.ny;
-  const long base = (long)o * a.npts;
-  double2 w1 = make_double2(0.0, 0.0), w2 = make_double2(0.0, 0.0), w3 = make_double2(0.0, 0.0);
-#pragma unroll
-  for (int s = 1; s <= ND; ++s) {
-    const long zp = base + p + (long)(wrapi(z + s, a.nz) - z) * sz, zm = base + p + (long)(wrapi(z - s, a.nz) - z) * sz;
-    const long yp = base + p + (long)(wrapi(y + s, a.ny) - y) * sy, ym = base + p + (long)(wrapi(y - s, a.ny) - y) * sy;
-    w1 = cadd(w1, cscal(n.nab[8 + s - 1], csub(__ldg(wy + zp), __ldg(wy + zm))));  // yz
-    w2 = cadd(w2, cscal(n.nab[8 + s - 1], csub(__ldg(wx + zp), __ldg(wx + zm))));  // zx
-    w3 = cadd(w3, cscal(n.nab[4 + s - 1], csub(__ldg(wx + yp), __ldg(wx + ym))));  // xy
-  }
-  const long gi = base + p;
-  const double2 mix = cadd(cadd(cscal(n.F[3], w1), cscal(n.F[4], w2)), cscal(n.F[5], w3));
-  double2 h = csub(__ldg(h1 + gi), cscal(0.5, mix));
-  if (a.nlma > 0) {
-    const int pm = __ldg(a.pmap + p);
-    if (pm >= 0) {
-      const int ik = o / a.nspin_no;
-      const double2* pj = a.proj + (long)o * a.nlma;
-      const double2* zk = a.ent_zk + (long)ik * a.nent;
-      const int e1 = (pm >> 8) + (pm & 255);
-      for (int e = pm >> 8; e < e1; ++e) h = cadd(h, cmul(pj[__ldg(a.ent_lma + e)], __ldg(zk + e)));
-    }
-  }
-  const double2 c = __ldg(in + gi);
-  if (MODE <= 2) hout[gi] = h;
-  if (MODE == 1 || MODE == 4) acc[gi] = cadd(c, cmul(a.zc, h));
-  if (MODE == 2 || MODE == 3) acc[gi] = cadd(acc[gi], cmul(a.zc, h));
-}
-
-// the scratch of the non-orthogonal hpsi (called before a graph capture, and by every launch)
-int nonorth_prepare(sb200_ctx* c) {
-  if (!c->g.nonorth) return SB200_OK;
-  const size_t need = 3 * (size_t)c->orb.norb * (size_t)c->g.npts;
-  if (c->nonorth_cap < need) {
-    dfree(c->d_nonorth);
-    c->nonorth_cap = 0;
-    if (dalloc(&c->d_nonorth, need) != SB200_OK) return SB200_ERR_OOM;
-    c->nonorth_cap = need;
-  }
-  return SB200_OK;
-}
-
-int launch_hpsi_nonorth(sb200_ctx* c, const HpsiLaunch& L) {
-  if (L.mode > 4) return set_error(SB200_ERR_UNSUPPORTED, "the non-orthogonal hpsi has no mixed-precision modes");
-  if (nonorth_prepare(c) != SB200_OK) return SB200_ERR_OOM;
-  const size_t blk = (size_t)c->orb.norb * (size_t)c->g.npts;
-  double2* h1 = c->d_nonorth;
-  double2* wx = h1 + blk;
-  double2* wy = wx + blk;
-  const HArgs a = make_hargs(c, L.zc);
-  NoArgs n;
-  for (int i = 0; i < 6; ++i) n.F[i] = c->g.coefF[i];
-  for (int i = 0; i < 12; ++i) n.nab[i] = c->g.coef_nab[i];
-  dim3 grid((unsigned)((c->g.npts + 255) / 256), c->orb.norb);
-  const double2* IN = (const double2*)L.in;
-  double2* HOUT = (double2*)L.hout;
-  k_hpsi_no1<<<grid, 256, 0, c->stream>>>(IN, h1, wx, wy, a, n);
-  switch (L.mode) {
-    case 0: k_hpsi_no2<0><<<grid, 256, 0, c->stream>>>(IN, h1, wx, wy, HOUT, L.out, a, n); break;
-    case 1: k_hpsi_no2<1><<<grid, 256, 0, c->stream>>>(IN, h1, wx, wy, HOUT, L.out, a, n); break;
-    case 2: k_hpsi_no2<2><<<grid, 256, 0, c->stream>>>(IN, h1, wx, wy, HOUT, L.out, a, n); break;
-    case 3: k_hpsi_no2<3><<<grid, 256, 0, c->stream>>>(IN, h1, wx, wy, HOUT, L.out, a, n); break;
-    default: k_hpsi_no2<4><<<grid, 256, 0, c->stream>>>(IN, h1, wx, wy, HOUT, L.out, a, n); break;
-  }
-  SB_LAUNCH_CHECK("k_hpsi_no1 / k_hpsi_no2");
-  return SB200_OK;
-}
 
 // ---------------------------------------------------------------------------
 // hpsi with a microscopic vector potential (single-scale Maxwell-TDDFT,
@@ -981,7 +846,6 @@ int launch_hpsi_micro(sb200_ctx* c, const HpsiLaunch& L) {
   if (L.mode > 4) return set_error(SB200_ERR_UNSUPPORTED, "the single-scale hpsi has no mixed-precision modes");
   const HArgs a = make_hargs(c, L.zc);
   NoArgs n;
-  for (int i = 0; i < 6; ++i) n.F[i] = 0.0;
   for (int i = 0; i < 12; ++i) n.nab[i] = c->g.coef_nab[i];
   dim3 grid((unsigned)((c->g.npts + 255) / 256), c->orb.norb);
   const double2* IN = (const double2*)L.in;
@@ -1210,7 +1074,6 @@ int launch_micro_current(sb200_ctx* c, const double2* psi, double* curr, double*
   micro_current_chunks(c, &pb, &nchunk, &nper);
   const HArgs a = make_hargs(c, make_double2(0.0, 0.0));
   NoArgs n;
-  for (int i = 0; i < 6; ++i) n.F[i] = 0.0;
   for (int i = 0; i < 12; ++i) n.nab[i] = c->g.coef_nab[i];
   k_micro_current<<<dim3((unsigned)pb, (unsigned)nchunk), dim3(32, 8), 0, c->stream>>>(psi, part, a, n, c->d_vec_k,
                                                                                       c->d_weight, c->orb.norb, nper);
