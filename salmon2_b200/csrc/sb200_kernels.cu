@@ -18,7 +18,7 @@ struct PrepArgs {
   int itt;                      // < 0: read *step
   double coef_lap0, coef_nab[12];
   const double* vec_k;          // [nk][3]
-  const double* A;              // a_mode 0: A[3]; 1, 2: Ac_tot(3, 0:nt+1); 3: Ac_ext
+  const double* A;              // a_mode 0: A[3] (4: Aval); 1, 2: Ac_tot(3, 0:nt+1); 3: Ac_ext
   const double* A2;             // a_mode 3: Ac_ind(3, 0:nt+1)
   const int* step;
   const double* pt_r;           // [totpts][3]
@@ -32,16 +32,18 @@ struct PrepArgs {
   const int* pair_fp;
   double2* pair_ph;             // [nk][npair] exp(i kAc.r), or null
   double rB[9];                 // rmatrix_B (identity on orthogonal cells)
+  double Aval[3];               // a_mode 4
 };
 
 __global__ void k_prep(PrepArgs a) {
   const int per = a.totpts > 0 ? a.totpts : 1;
   const long items = (long)a.nk * per;
   int itt = a.itt;
-  if (a.a_mode != 0 && itt < 0) itt = *a.step;
+  if (a.a_mode != 0 && a.a_mode != 4 && itt < 0) itt = *a.step;
   double A[3];
   for (int d = 0; d < 3; ++d) {
-    if (a.a_mode == 0) A[d] = a.A[d];
+    if (a.a_mode == 4) A[d] = a.Aval[d];
+    else if (a.a_mode == 0) A[d] = a.A[d];
     else if (a.a_mode == 1) A[d] = 0.5 * (a.A[3 * itt + d] + a.A[3 * (itt - 1) + d]);
     else if (a.a_mode == 2) A[d] = a.A[3 * itt + d];
     else  // the AETRS prediction of A(itt+1), time_evolution_step.f90:466-470
@@ -573,6 +575,7 @@ int launch_prep_k(sb200_ctx* c, const double* d_A, int a_mode, int itt, double* 
   a.pair_fp = c->pp.d_pair_fp;
   a.pair_ph = (phases && c->g.periodic && c->pp.npair > 0) ? c->pp.d_pair_ph : nullptr;
   for (int i = 0; i < 9; ++i) a.rB[i] = c->g.rB[i];
+  for (int d = 0; d < 3; ++d) a.Aval[d] = c->vec_Ac[d];
   long items = (long)a.nk * (a.totpts > 0 ? a.totpts : 1);
   if ((long)a.nk * a.nent > items) items = (long)a.nk * a.nent;
   if ((long)a.nk * a.npair > items) items = (long)a.nk * a.npair;
