@@ -1326,20 +1326,25 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
   }
   SB_CUDA(cudaStreamSynchronize(c->stream));
 
-  // Two steps (A->B, B->A) captured as one CUDA graph and replayed.
+  // The first step (nt odd) or two are launched one by one: the device works on
+  // them while the rest, two steps (A->B, B->A) at a time, is captured as one
+  // CUDA graph, instantiated and replayed.  (With all steps in the graph the
+  // device waited for it, 100 to 130 us a call.)
   cudaGraphExec_t exec2 = nullptr;
-  const int pairs = c->timing ? 0 : nt / 2;
   int rc = SB200_OK;
   // with AETRS every step maps A -> A (B its half-step scratch)
   double2* A2 = c->aetrs ? A : B;
   double2* B2 = c->aetrs ? B : A;
-  if (c->timing) {  // instrumented: every launch bracketed by events, no graph
-    for (int i = 0; i + 1 < nt; i += 2) {
-      TRY(issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt));
-      TRY(timing_flush(c));
-      TRY(issue_rt_step(c, A2, B2, W, z.data(), n_hamil, trans_longi, dt));
-      TRY(timing_flush(c));
-    }
+  const int lead = c->timing ? nt : (nt % 2 == 1 ? 1 : std::min(nt, 2));
+  for (int i = 0; i < lead; ++i) {  // instrumented: every step, its launches bracketed by events
+    TRY(i % 2 == 0 ? issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt)
+                   : issue_rt_step(c, A2, B2, W, z.data(), n_hamil, trans_longi, dt));
+    if (c->timing) TRY(timing_flush(c));
+  }
+  const int pairs = (nt - lead) / 2;
+  if (lead % 2 == 1) {  // the graph starts from the odd step's result
+    std::swap(A, A2);
+    std::swap(B, B2);
   }
   if (pairs > 0) {
     cudaGraph_t graph = nullptr;
@@ -1362,11 +1367,7 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
     cudaGraphExecDestroy(exec2);
     if (rc != SB200_OK) return rc;
   }
-  double2* final_buf = A;
-  if (nt % 2 == 1) {
-    TRY(issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt));
-    final_buf = c->aetrs ? A : B;
-  }
+  double2* final_buf = nt % 2 == 1 && !c->aetrs ? (double2*)psi_b : (double2*)psi_a;
   if (curr_out && nt > 0)
     SB_CUDA(cudaMemcpyAsync(curr_out, r.d_curr, 3 * (size_t)nt * sizeof(double), cudaMemcpyDefault, c->stream));
   if (rbox_out && nt > 0)
