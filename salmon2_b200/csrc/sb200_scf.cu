@@ -17,10 +17,12 @@
 // does not depend on the launch shape.  The grids of this path (16^3 to 128^3)
 // make each pass a few microseconds to tens of microseconds; the tables
 // (3 n^2 complex) and 4 pi / |G|^2 stay resident across steps.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 #include <nccl.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -28,6 +30,8 @@
 #include <vector>
 
 #include "sb200_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace sb200 {
 namespace {
@@ -404,6 +408,109 @@ __global__ void __launch_bounds__(SCF_DFT_THREADS) k_dft_pass(const double2* __r
   }
 }
 
+// The six passes in one launch, a cluster of eight CTAs: CTA r holds the x slab
+// r nx / 8 .. and makes the z and y passes on it; every CTA then gathers an eighth
+// of the x lines from the slabs, transforms them, multiplies by coef / ntot,
+// transforms back (the inverse x pass first: the axes commute), and the owners
+// gather their slabs for the inverse z and y passes.  Six launches of k_dft_pass
+// are bound by launch and load latency on small grids: 16^3 27 us and the gaps
+// between them, here 11 us (21 with the tables read through L1: cold at each launch).
+// A thread forms DFT_K outputs of a line, so a value is read once for them, and
+// the lanes of a warp take neighbouring lines, so a table entry is one broadcast;
+// each pass writes the layout whose lines the next one reads side by side.
+constexpr int DFT_CTAS = 8, DFT_NT = 512, DFT_K = 2;
+
+// out(u, k) = sum_j T(k, j) in[u + nu j] for nu lines of length n, through put(u, k, sum)
+template <typename Put>
+__device__ __forceinline__ void dft_lines(const double2* in, int nu, int n, const double2* T, double sg,
+                                          Put put) {
+  const int groups = (n + DFT_K - 1) / DFT_K;
+  for (int i = threadIdx.x; i < nu * groups; i += DFT_NT) {
+    const int u = i % nu, k0 = (i / nu) * DFT_K;
+    double re[DFT_K], im[DFT_K];
+    const double2* Tk[DFT_K];
+#pragma unroll
+    for (int q = 0; q < DFT_K; ++q) {
+      re[q] = im[q] = 0.0;
+      Tk[q] = T + (long)min(k0 + q, n - 1) * n;
+    }
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+      const double2 v = in[u + nu * j];
+#pragma unroll
+      for (int q = 0; q < DFT_K; ++q) {
+        const double2 t = Tk[q][j];
+        const double ti = sg * t.y;
+        re[q] = re[q] + (t.x * v.x - ti * v.y);
+        im[q] = im[q] + (t.x * v.y + ti * v.x);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < DFT_K; ++q)
+      if (k0 + q < n) put(u, k0 + q, make_double2(re[q], im[q]));
+  }
+}
+
+__global__ void __cluster_dims__(DFT_CTAS, 1, 1) __launch_bounds__(DFT_NT, 1)
+    k_hartree_cluster(const double* __restrict__ rho, double* __restrict__ vh, const double2* __restrict__ tab,
+                      const double* __restrict__ coef, int nx, int ny, int nz, int cap) {
+  extern __shared__ __align__(16) double2 db[];
+  double2 *b0 = db, *b1 = db + cap, *b2 = db + 2 * cap;
+  double2 *tx = db + 3 * cap, *ty = tx + nx * nx, *tz = ty + ny * ny;  // the tables of the axes, one after the other
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), t = threadIdx.x;
+  const int nyz = ny * nz;
+  const int x0 = rank * nx / DFT_CTAS, xs = (rank + 1) * nx / DFT_CTAS - x0;
+  const int l0 = rank * nyz / DFT_CTAS, nl = (rank + 1) * nyz / DFT_CTAS - l0;
+  const int slab = xs * nyz;
+  for (int i = t; i < nx * nx + ny * ny + nz * nz; i += DFT_NT) tx[i] = __ldg(tab + i);
+  for (int i = t; i < slab; i += DFT_NT)  // (x, y) lines along z
+    b0[i] = make_double2(__ldg(rho + x0 + i % xs + (long)nx * (i / xs)), 0.0);
+  __syncthreads();
+  dft_lines(b0, xs * ny, nz, tz, -1.0,
+            [&](int u, int k, double2 v) { b1[u % xs + xs * (k + nz * (u / xs))] = v; });  // (x, z) lines along y
+  __syncthreads();
+  dft_lines(b1, xs * nz, ny, ty, -1.0,
+            [&](int u, int k, double2 v) { b0[(u % xs) * nyz + k + ny * (u / xs)] = v; });  // by x, then y + ny z
+  cl.sync();
+  for (int i = t; i < nl * nx; i += DFT_NT) {  // this CTA's x lines
+    const int u = i % nl, x = i / nl;
+    const int o = ((x + 1) * DFT_CTAS - 1) / nx, xl = x - o * nx / DFT_CTAS;  // owner: the last slab that starts at or below x
+    b1[i] = cl.map_shared_rank(b0, o)[xl * nyz + l0 + u];
+  }
+  __syncthreads();
+  const double ntot = (double)nx * nyz;
+  dft_lines(b1, nl, nx, tx, -1.0, [&](int u, int k, double2 v) {
+    const double cf = __ldg(coef + k + (long)nx * (l0 + u));
+    b2[u + nl * k] = make_double2(cf * (v.x / ntot), cf * (v.y / ntot));
+  });
+  __syncthreads();
+  dft_lines(b2, nl, nx, tx, 1.0, [&](int u, int k, double2 v) { b1[u + nl * k] = v; });
+  cl.sync();
+  for (int i = t; i < slab; i += DFT_NT) {
+    const int l = i % nyz, xl = i / nyz;
+    const int o = ((l + 1) * DFT_CTAS - 1) / nyz, lo = o * nyz / DFT_CTAS, no = (o + 1) * nyz / DFT_CTAS - lo;
+    b0[xl + xs * l] = cl.map_shared_rank(b1, o)[l - lo + no * (x0 + xl)];
+  }
+  cl.sync();  // the slabs are there; every CTA is done with the others' shared memory
+  dft_lines(b0, xs * ny, nz, tz, 1.0,
+            [&](int u, int k, double2 v) { b2[u % xs + xs * (k + nz * (u / xs))] = v; });
+  __syncthreads();
+  dft_lines(b2, xs * nz, ny, ty, 1.0,
+            [&](int u, int k, double2 v) { vh[x0 + u % xs + (long)nx * (k + (long)ny * (u / xs))] = v.x; });
+}
+
+// Elements of one of the three buffers of the form above, 0: six launches.  Eight
+// SMs make a pass in about npts n / 128 cycles, where a launch with its load
+// latency is 5 us: the line lies where those meet, n of about 24 on a cube.
+long hartree_cluster_cap(int nx, int ny, int nz) {
+  const long n = (long)nx * ny * nz;
+  if (n * (nx + ny + nz) > 1100000L) return 0;
+  const long slab = (long)((nx + DFT_CTAS - 1) / DFT_CTAS) * ny * nz;
+  const long share = ((long)ny * nz + DFT_CTAS - 1) / DFT_CTAS * nx;
+  return std::max(slab, share);
+}
+
 // One pass of the isolated solve on the doubled (mx, my, mz) box: outputs on
 // the corner box [0,bx) x [0,by) x [0,bz), each the ordered sum over the first
 // nsum inputs along `axis` of T(k, j) * in(j), T the exp(+-2 pi i jk / ma) table
@@ -581,6 +688,15 @@ int scf_launch_hartree(sb200_ctx* c, const double* d_rho, double* d_vh, int kind
   const double2* tx = s->d_tab;
   const double2* ty = tx + (size_t)nx * nx;
   const double2* tz = ty + (size_t)ny * ny;
+  const long cap = hartree_cluster_cap(nx, ny, nz);
+  const size_t smem = (3 * (size_t)cap + (size_t)nx * nx + (size_t)ny * ny + (size_t)nz * nz) * sizeof(double2);
+  if (cap > 0 && smem <= 200u * 1024u) {
+    SB_CUDA(cudaFuncSetAttribute(k_hartree_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TRY_S(scf_mark(c, kind, true));
+    k_hartree_cluster<<<DFT_CTAS, DFT_NT, smem, c->stream>>>(d_rho, d_vh, tx, s->d_coef, nx, ny, nz, (int)cap);
+    TRY_S(scf_mark(c, kind, false));
+    return SB200_OK;
+  }
   long gbl = (n + SCF_DFT_THREADS - 1) / SCF_DFT_THREADS;
   if (gbl > 148L * 16) gbl = 148L * 16;
   const int gb = (int)gbl;
