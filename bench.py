@@ -208,13 +208,14 @@ def orbital_path(s, args):
     return s.grid.periodic and tuple(s.grid.shape) == (16, 16, 16) and args.precision == "fp64"
 
 
-def hpsi_kernel(s, args, units_per_launch):
+def hpsi_kernel(s, args, units_per_launch, per_step):
     """(name, algorithmic bytes per launch) of the kernel that applies H.
 
     The algorithmic bytes of a Taylor step are 224 B per unit (FP64; 144 B
     mixed) whatever the kernel split: a per-term kernel is credited a quarter
     per launch, the fused-step kernel (all four terms in one launch, which
-    itself moves only psi in and psi_out out) the whole 224 B."""
+    itself moves only psi in and psi_out out) the whole 224 B.
+    per_step: its launches in a time step."""
     if orbital_path(s, args):
         v = os.environ.get("SB200_ORBITAL", "fused")
         if v.startswith("p"):
@@ -226,6 +227,8 @@ def hpsi_kernel(s, args, units_per_launch):
         if v.startswith("s"):
             return "k_step_orbital_st", UNIT_BYTES["fp64"] * units_per_launch  # KB tables in shared memory
         return "k_step_blk", UNIT_BYTES["fp64"] * units_per_launch  # register-blocked fused step
+    if per_step == 1:
+        return "k_step_any", UNIT_BYTES[args.precision] * units_per_launch  # fused step in a cluster
     name = "k_hpsi_tiled" if os.environ.get("SB200_TMA", "on").startswith("of") else "k_hpsi_tma"
     return name, UNIT_BYTES[args.precision] / 4.0 * units_per_launch
 
@@ -276,11 +279,13 @@ def supercell_leg(args, local):
         kt = ctx.kernel_times(reset=True)
         ctx.set_timing(False)
         h_ms, h_cnt = kt.get("hpsi", (float("nan"), 1))
-        bytes_launch = UNIT_BYTES[prec] / 4.0 * units / nt
+        fused = h_cnt == min(nt, 20)  # one launch a step: the cluster form; else one a term
+        kernel = "k_step_any" if fused else "k_hpsi_tma"
+        bytes_launch = UNIT_BYTES[prec] / (1.0 if fused else 4.0) * units / nt
         ach = bytes_launch / (h_ms / h_cnt / 1e3) / 1e9
-        out[prec] = {"value": value, "kernel": "k_hpsi_tma", "avg_launch_ms": h_ms / h_cnt,
+        out[prec] = {"value": value, "kernel": kernel, "avg_launch_ms": h_ms / h_cnt,
                      "algorithmic_bytes_per_launch": bytes_launch, "achieved_gbs": ach, "frac": ach / peak,
-                     "traffic": ncu_traffic("k_hpsi_tma", "supercell") if prec == "fp64" else None}
+                     "traffic": ncu_traffic(kernel, "supercell") if prec == "fp64" else None}
         ctx.close()
         del a, b, w, psi0
         torch.cuda.empty_cache()
@@ -673,9 +678,9 @@ def main():
     launches_per_tstep = sum(v[1] for v in kt.values()) / nt_i
     gpu_launches = int(round(launches_per_tstep * nt * args.steps))
     units_per_launch = int(np.prod(s.grid.shape)) * s.norb
-    kname, bytes_per_launch = hpsi_kernel(s, args, units_per_launch)
-    peak, peak_kind = measured_peaks()
     h_ms, h_cnt = kt.get("hpsi", (float("nan"), 1))
+    kname, bytes_per_launch = hpsi_kernel(s, args, units_per_launch, h_cnt / nt_i)
+    peak, peak_kind = measured_peaks()
     avg_ms = h_ms / h_cnt
     achieved = bytes_per_launch / (avg_ms / 1e3) / 1e9
     traffic = ncu_traffic(kname, args.workload)
