@@ -1329,7 +1329,7 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
   // The first step (nt odd) or two are launched one by one: the device works on
   // them while the rest, two steps (A->B, B->A) at a time, is captured as one
   // CUDA graph, instantiated and replayed.  (With all steps in the graph the
-  // device waited for it, 100 to 130 us a call.)
+  // device waited for it, 65 to 75 us a call.)
   cudaGraphExec_t exec2 = nullptr;
   int rc = SB200_OK;
   // with AETRS every step maps A -> A (B its half-step scratch)
