@@ -921,6 +921,7 @@ cudaError_t launch_solve(const PArgs& a, int grid, cudaStream_t st) { return lau
 
 // own and halo points a thread of k_pcg_box can hold, by instantiation
 constexpr int BOX_MO[3] = {2, 4, 6}, BOX_MH[3] = {5, 8, 11};
+constexpr int BOX_STATIC = 1024;  // room for the kernel's static shared memory
 int box_which(const Boxes& b) {
   for (int i = 0; i < 3; ++i)
     if (b.own <= BOX_MO[i] * BXT && b.halo <= BOX_MH[i] * BXT) return i;
@@ -966,7 +967,7 @@ Boxes boxes_for(int nx, int ny, int nz, int device) {
       b.own = bx * by * bz;
       b.halo = 2 * HALO * (by * bz + bx * bz + bx * by);
       b.smem = (size_t)(bx + 2 * HALO) * (by + 2 * HALO) * (bz + 2 * HALO) * sizeof(double);
-      if (box_which(b) < 0 || b.smem + 1024 > (size_t)optin) continue;
+      if (box_which(b) < 0 || b.smem > (size_t)(optin - BOX_STATIC)) continue;
       const double w = b.own + b.halo / 3.0;
       if (best.g[0] == 0 || w < cost) {
         cost = w;
@@ -974,9 +975,11 @@ Boxes boxes_for(int nx, int ny, int nz, int device) {
       }
     }
   if (best.g[0] == 0) return best;
+  // the limit belongs to the function, not to this context: the largest any box may
+  // take, so that another context's smaller box leaves this one's launches alone
   const void* k = box_kernel(box_which(best));
   int per_sm = 0;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best.smem) != cudaSuccess ||
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - BOX_STATIC) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, BXT, best.smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return Boxes();
