@@ -39,6 +39,7 @@ constexpr int MAX_NT = 256;  // two CTAs an SM, 128 registers a thread (112 spil
 constexpr int REGS = 128;
 constexpr int RING = 4;      // planes resident or in flight
 constexpr int SLOTS = 4;     // plane values a thread copies at most
+constexpr int SMEM_LIMIT = 200 * 1024;  // of every tile: the kernel's limit is shared by all contexts
 
 struct NoArgs {
   int w, h;  // tile
@@ -231,7 +232,7 @@ NonorthTile tile_shape(const GridInfo& g, int norb) {
       k.smem = ((size_t)RING * area + 2 * (size_t)(w + 2 * ND) * h) * sizeof(double2);
       if (k.NT > MAX_NT) continue;
       const long tiles = (long)((g.nx + w - 1) / w) * ((g.ny + h - 1) / h);
-      const int per_sm = std::min(std::min(32, 65536 / (REGS * k.NT)), (int)(200 * 1024 / k.smem));
+      const int per_sm = std::min(std::min(32, 65536 / (REGS * k.NT)), (int)(SMEM_LIMIT / k.smem));
       for (k.nchunk = 1; k.nchunk <= 16 && (k.nchunk == 1 || g.nz / k.nchunk >= 4); ++k.nchunk) {
         const int zc = (g.nz + k.nchunk - 1) / k.nchunk, nzc = (g.nz + zc - 1) / zc;
         const long ctas = tiles * norb * nzc, slots = 148L * per_sm;
@@ -249,7 +250,7 @@ NonorthTile tile_shape(const GridInfo& g, int norb) {
 
 template <int MODE>
 int launch_mode(const HpsiLaunch& L, const TiledArgs& a, const NoArgs& n, const NonorthTile& k, dim3 grid, cudaStream_t st) {
-  SB_CUDA(cudaFuncSetAttribute(k_hpsi_no<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
+  SB_CUDA(cudaFuncSetAttribute(k_hpsi_no<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
   k_hpsi_no<MODE><<<grid, k.NT, k.smem, st>>>((const double2*)L.in, (double2*)L.hout, L.out, a, n);
   SB_LAUNCH_CHECK("k_hpsi_no");
   return SB200_OK;

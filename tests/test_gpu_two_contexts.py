@@ -1,6 +1,8 @@
 """Contexts of different grids side by side, as two systems in one program: what
 one of them sets up or launches leaves the other's launches alone (limits of a
 kernel that belong to the function, not to the context)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -36,3 +38,36 @@ def test_cg_hartree_of_two_box_sizes():
     assert np.array_equal(loop(first), ref)
     first.close()
     second.close()
+
+
+def _together(jobs):
+    """Every job in a host thread of its own (one context each); the first error."""
+    errors = []
+
+    def guarded(job):
+        try:
+            job()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=guarded, args=(j,)) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
+
+
+def test_nonorthogonal_grids_in_two_threads():
+    """H psi on two lattices whose tiles take 20 and 40 KB, each from its own
+    host thread: no launch is refused and the results stay right."""
+    from salmon2_b200.rt import Context
+    cell = np.array([[0.60, 0.0, 0.0], [0.16, 0.57, 0.0], [-0.09, 0.19, 0.66]]).T
+    systems = [synth.nonorthogonal_system(cell * np.array(n), n, nkgrid=1, no=1, seed=sum(n), natom=1)
+               for n in ((8, 8, 8), (24, 24, 20))]
+    ctxs = [Context(s) for s in systems]
+    bufs = [(c.upload(s.psi), c.zeros()) for c, s in zip(ctxs, systems)]
+    _together([lambda c=c, b=b: [c.hpsi(*b) for _ in range(3000)] for c, b in zip(ctxs, bufs)])
+    for c, s, b in zip(ctxs, systems, bufs):
+        assert S.rel_err(c.download(b[1]), Oracle(s).hpsi(s.psi)) < 1e-12
+        c.close()
