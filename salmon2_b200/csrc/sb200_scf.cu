@@ -419,6 +419,7 @@ __global__ void __launch_bounds__(SCF_DFT_THREADS) k_dft_pass(const double2* __r
 // the lanes of a warp take neighbouring lines, so a table entry is one broadcast;
 // each pass writes the layout whose lines the next one reads side by side.
 constexpr int DFT_CTAS = 8, DFT_NT = 512, DFT_K = 2;
+constexpr int DFT_SMEM = 200 * 1024;  // most shared memory of a CTA
 
 // out(u, k) = sum_j T(k, j) in[u + nu j] for nu lines of length n, through put(u, k, sum)
 template <typename Put>
@@ -690,10 +691,12 @@ int scf_launch_hartree(sb200_ctx* c, const double* d_rho, double* d_vh, int kind
   const double2* tz = ty + (size_t)ny * ny;
   const long cap = hartree_cluster_cap(nx, ny, nz);
   const size_t smem = (3 * (size_t)cap + (size_t)nx * nx + (size_t)ny * ny + (size_t)nz * nz) * sizeof(double2);
-  if (cap > 0 && smem <= 200u * 1024u) {
-    SB_CUDA(cudaFuncSetAttribute(k_hartree_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (cap > 0 && smem <= (size_t)DFT_SMEM) {
+    // (the same for every grid: the limit is shared by all contexts)
+    SB_CUDA(cudaFuncSetAttribute(k_hartree_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, DFT_SMEM));
     TRY_S(scf_mark(c, kind, true));
     k_hartree_cluster<<<DFT_CTAS, DFT_NT, smem, c->stream>>>(d_rho, d_vh, tx, s->d_coef, nx, ny, nz, (int)cap);
+    SB_LAUNCH_CHECK("k_hartree_cluster");
     TRY_S(scf_mark(c, kind, false));
     return SB200_OK;
   }

@@ -71,3 +71,19 @@ def test_nonorthogonal_grids_in_two_threads():
     for c, s, b in zip(ctxs, systems, bufs):
         assert S.rel_err(c.download(b[1]), Oracle(s).hpsi(s.psi)) < 1e-12
         c.close()
+
+
+def test_periodic_hartree_in_two_threads():
+    """The one-launch periodic Hartree solve of 8^3 and 24^3 grids (6 and 108 KB a
+    CTA), each from its own host thread, against the oracle."""
+    import oracle as OR
+    from salmon2_b200.rt import Context
+    rng, jobs = np.random.default_rng(4), []
+    for n in (8, 24):
+        s = synth.periodic_system(a=10.26, num=n, nkgrid=1, no=1, seed=n)
+        brl = OR.primitive_b_orthogonal([m * h for m, h in zip(s.grid.shape, s.grid.hgs)])
+        jobs.append((Context(s), rng.uniform(0.0, 0.2, s.grid.shape), brl))
+    _together([lambda c=c, r=r, b=b: [c.hartree_periodic(r, b) for _ in range(800)] for c, r, b in jobs])
+    for c, r, b in jobs:
+        assert S.rel_err(c.hartree_periodic(r, b), OR.poisson_ft(r, b)) < 1e-12
+        c.close()
