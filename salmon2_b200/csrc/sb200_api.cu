@@ -585,7 +585,8 @@ int sb200_set_grid(sb200_ctx* c, const int is[3], const int ie[3], const int is_
     g.coef_nab[i] = coef_nab[i];
   }
   g.set = true;
-  const bool changed = !c->g.set || c->g.npts != g.npts || c->g.periodic != g.periodic;
+  // (the projector tables hold planes and linear indices of these extents)
+  const bool changed = !c->g.set || c->g.nx != g.nx || c->g.ny != g.ny || c->g.nz != g.nz || c->g.periodic != g.periodic;
   c->g = g;
   if (changed) {
     // tables that depend on the grid must be provided again

@@ -1,0 +1,66 @@
+"""A context whose grid or orbitals are set again: tables of the earlier shape are
+never used with the new one, and a context set up in steps computes what a
+fresh one does."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import _systems as S
+from oracle import Oracle
+from salmon2_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+_dp, _ip = C.POINTER(C.c_double), C.POINTER(C.c_int)
+
+
+def _set_grid(ctx, g):
+    from salmon2_b200._lib import check, lib
+    i3 = lambda v: (C.c_int * 3)(*[int(x) for x in v])  # noqa: E731
+    maps = [np.ascontiguousarray(a, dtype=np.int32) for a in (g.idx, g.idy, g.idz)]
+    lap, nab = (np.ascontiguousarray(np.asarray(a).ravel(order="F")) for a in (g.coef_lap, g.coef_nab))
+    hgs = np.ascontiguousarray(g.hgs, dtype=np.float64)
+    check(lib().sb200_set_grid(ctx.h, i3(g.is_), i3(g.ie), i3(g.is_array), i3(g.ie_array),
+                               *[m.ctypes.data_as(_ip) for m in maps], i3(g.num), hgs.ctypes.data_as(_dp), g.hvol,
+                               g.coef_lap0, lap.ctypes.data_as(_dp), nab.ctypes.data_as(_dp)))
+
+
+def _set_vlocal(ctx, V):
+    from salmon2_b200._lib import check, lib
+    v = np.asfortranarray(V, dtype=np.float64)
+    check(lib().sb200_set_vlocal(ctx.h, v.ctypes.data_as(_dp)))
+
+
+def _cell(num):
+    cell = 0.62 * np.array(num)
+    rng = np.random.default_rng(sum(num))
+    grid = synth.make_grid(np.array(num), cell / np.array(num), periodic=True)
+    rion = np.asfortranarray(rng.uniform(0.0, 1.0, (3, 3)) * cell[:, None])
+    V = synth.gaussian_potential(grid, rion, np.full(3, -1.0), np.full(3, 1.0), cell=cell)
+    pp = synth.make_pp(grid, rion, 2.2, sigma=0.6, amp=0.4, inorm=np.ones((3, 2), dtype=int), cell=cell)
+    vec_k, wtk = synth.mp_kpoints(1, cell)
+    return synth.System(grid, pp, 1, 2, 1, vec_k, np.full((2, 1, 1), 2.0, order="F"), wtk,
+                        np.asfortranarray(V[..., None]), rion, synth.random_orbitals(grid, rng, 1, 2, 1),
+                        int(np.prod(num)), 1)
+
+
+def test_grid_of_as_many_points_and_other_extents():
+    """12 x 24 x 12 -> 12 x 12 x 24 points: V_local and the projectors of the first
+    grid are gone (H psi is refused), and right once they are set again."""
+    from salmon2_b200._lib import SB200Error
+    from salmon2_b200.rt import Context
+    first, second = _cell((12, 24, 12)), _cell((12, 12, 24))
+    ctx = Context(first)
+    psi, out = ctx.upload(first.psi), ctx.zeros()
+    ctx.hpsi(psi, out)
+    _set_grid(ctx, second.grid)
+    with pytest.raises(SB200Error):
+        ctx.hpsi(psi, out)
+    _set_vlocal(ctx, second.V_local)
+    bare = S.no_pp(second)
+    ctx.sys, ctx.shape = second, (second.norb,) + second.grid.shape[::-1]
+    assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(second.psi), ctx.zeros())), Oracle(bare).hpsi(second.psi)) < 1e-12
+    ctx.set_pp(second.pp)
+    assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(second.psi), ctx.zeros())), Oracle(second).hpsi(second.psi)) < 1e-12
+    ctx.close()
