@@ -594,6 +594,11 @@ int sb200_set_grid(sb200_ctx* c, const int is[3], const int ie[3], const int is_
     dfree(c->d_vloc);
     dfree(c->d_vloc32);
     c->vloc_set = false;
+    dfree(c->d_cap);
+    c->cap_on = 0;
+    dfree(c->d_acm);
+    dfree(c->d_divac);
+    c->microac = 0;
   }
   TRY(ensure_work(c));
   TRY(refresh_k(c));

@@ -64,3 +64,27 @@ def test_grid_of_as_many_points_and_other_extents():
     ctx.set_pp(second.pp)
     assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(second.psi), ctx.zeros())), Oracle(second).hpsi(second.psi)) < 1e-12
     ctx.close()
+
+
+@pytest.mark.parametrize("extra", ["absorbing", "microscopic"])
+def test_fields_of_the_earlier_grid(extra):
+    """The absorbing boundary's plane table and the microscopic vector potential of
+    a smaller grid go with it, as V_local does: H psi of the larger grid is that
+    of a fresh context."""
+    from salmon2_b200.rt import Context
+    first, second = _cell((12, 12, 12)), _cell((12, 14, 40))
+    ctx = Context(first)
+    if extra == "absorbing":
+        ctx.set_absorbing_boundary(w0=0.3, dr=2.0)
+    else:
+        ctx.set_micro_ac(0.01 * np.ones((3,) + first.grid.shape, order="F"))
+    ctx.hpsi(ctx.upload(first.psi), ctx.zeros())
+    _set_grid(ctx, second.grid)
+    _set_vlocal(ctx, second.V_local)
+    ctx.sys, ctx.shape = second, (second.norb,) + second.grid.shape[::-1]
+    ctx.set_pp(second.pp)
+    assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(second.psi), ctx.zeros())), Oracle(second).hpsi(second.psi)) < 1e-12
+    if extra == "microscopic":  # a field of the new size is taken, and taken off again
+        ctx.set_micro_ac(0.01 * np.ones((3,) + second.grid.shape, order="F"))
+        ctx.set_micro_ac(None)
+    ctx.close()
