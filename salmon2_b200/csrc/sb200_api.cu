@@ -640,6 +640,10 @@ int sb200_set_orbitals(sb200_ctx* c, int nspin, int no, int nk, const double* ve
     c->pp.nk_phase = nk;
     TRY(dalloc(&c->pp.d_phase, (size_t)nk * c->pp.totpts));
     TRY(dalloc(&c->pp.d_ent_zk, (size_t)nk * (c->pp.nent > 0 ? c->pp.nent : 1)));
+    if (c->pp.d_pair_ph) {
+      dfree(c->pp.d_pair_ph);
+      TRY(dalloc(&c->pp.d_pair_ph, (size_t)nk * (c->pp.npair > 0 ? c->pp.npair : 1)));
+    }
   }
   TRY(ensure_work(c));
   TRY(refresh_k(c));

@@ -2,6 +2,7 @@
 never used with the new one, and a context set up in steps computes what a
 fresh one does."""
 import ctypes as C
+import dataclasses
 
 import numpy as np
 import pytest
@@ -30,6 +31,14 @@ def _set_vlocal(ctx, V):
     from salmon2_b200._lib import check, lib
     v = np.asfortranarray(V, dtype=np.float64)
     check(lib().sb200_set_vlocal(ctx.h, v.ctypes.data_as(_dp)))
+
+
+def _set_orbitals(ctx, s):
+    from salmon2_b200._lib import check, lib
+    k, occ = np.asfortranarray(s.vec_k, dtype=np.float64), np.asfortranarray(s.rocc, dtype=np.float64)
+    w = np.ascontiguousarray(s.wtk, dtype=np.float64)
+    check(lib().sb200_set_orbitals(ctx.h, s.nspin, s.no, s.nk, *[a.ctypes.data_as(_dp) for a in (k, occ, w)]))
+    ctx.sys, ctx.shape = s, (s.norb,) + s.grid.shape[::-1]
 
 
 def _cell(num):
@@ -87,4 +96,26 @@ def test_fields_of_the_earlier_grid(extra):
     if extra == "microscopic":  # a field of the new size is taken, and taken off again
         ctx.set_micro_ac(0.01 * np.ones((3,) + second.grid.shape, order="F"))
         ctx.set_micro_ac(None)
+    ctx.close()
+
+
+@pytest.mark.parametrize("num", [(12, 13, 14), (16, 16, 16)], ids=["cluster", "16cubed"])
+def test_more_k_points_after_the_projectors(num):
+    """One k-point, the projectors, then eight k-points: every phase table follows."""
+    from salmon2_b200.rt import Context
+    one = _cell(num)
+    vec_k, wtk = synth.mp_kpoints(2, 0.62 * np.array(num))
+    nk = vec_k.shape[1]
+    psi = synth.random_orbitals(one.grid, np.random.default_rng(5), 1, 2, nk)
+    many = dataclasses.replace(one, nk=nk, vec_k=vec_k, wtk=wtk, rocc=np.full((2, nk, 1), 2.0, order="F"), psi=psi)
+    ctx = Context(one)
+    _set_orbitals(ctx, many)
+    O = Oracle(many)
+    ac = (0.01, -0.02, 0.03)
+    O.set_vec_Ac(ac)
+    ctx.set_vec_Ac(ac)
+    assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(many.psi), ctx.zeros())), O.hpsi(many.psi)) < 1e-12
+    zc = synth.taylor_zc(0.03)
+    got = ctx.taylor(ctx.upload(many.psi), ctx.zeros(), ctx.zeros(), zc)
+    assert S.rel_err(ctx.download(got), O.taylor(many.psi, zc)) < 1e-12
     ctx.close()
