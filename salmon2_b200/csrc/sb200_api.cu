@@ -613,6 +613,11 @@ int sb200_set_orbitals(sb200_ctx* c, int nspin, int no, int nk, const double* ve
   DeviceGuard dg(c->device);
   OrbInfo& o = c->orb;
   const bool nk_changed = o.nk != nk;
+  if (c->d_vloc && nspin > c->vloc_nspin) {  // V_local has no second spin: it must be provided again
+    dfree(c->d_vloc);
+    dfree(c->d_vloc32);
+    c->vloc_set = false;
+  }
   o.nspin = nspin;
   o.no = no;
   o.nk = nk;
@@ -656,7 +661,10 @@ int sb200_set_vlocal(sb200_ctx* c, const double* V_local) {
   if (!V_local) return set_error(SB200_ERR_INVALID_ARG, "null V_local");
   DeviceGuard dg(c->device);
   const size_t n = (size_t)c->g.npts * c->orb.nspin;
-  if (!c->d_vloc) TRY(dalloc(&c->d_vloc, n));
+  if (!c->d_vloc) {
+    TRY(dalloc(&c->d_vloc, n));
+    c->vloc_nspin = c->orb.nspin;
+  }
   SB_CUDA(cudaMemcpy(c->d_vloc, V_local, n * sizeof(double), cudaMemcpyDefault));
   if (!c->d_vloc32) TRY(dalloc(&c->d_vloc32, n));
   std::vector<float> v32(n);

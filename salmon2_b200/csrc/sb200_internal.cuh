@@ -178,6 +178,7 @@ struct sb200_ctx {
   void* d_stage = nullptr;      // relayout staging
   size_t stage_bytes = 0;
   bool vloc_set = false;
+  int vloc_nspin = 0;          // spins d_vloc and d_vloc32 have room for
   NonorthTile no_tile;
   int any_C = -1;              // cluster size of the fused step of general periodic grids (0: does not apply,
                                // -1: to be chosen at the next step)

@@ -1045,7 +1045,10 @@ int sb200_update_vlocal(sb200_ctx* c, const double* Vpsl, const double* Vh, cons
   ScfState* s = scf_of(c);
   const long n = s->npts;
   const int nspin = c->orb.nspin;
-  if (!c->d_vloc) TRY_S(dalloc(&c->d_vloc, (size_t)n * nspin));
+  if (!c->d_vloc) {
+    TRY_S(dalloc(&c->d_vloc, (size_t)n * nspin));
+    c->vloc_nspin = nspin;
+  }
   if (!c->d_vloc32) TRY_S(dalloc(&c->d_vloc32, (size_t)n * nspin));
   TRY_S(scf_stage_in(c, (size_t)n * (2 + nspin)));
   const double *a = nullptr, *b = nullptr, *x = nullptr;

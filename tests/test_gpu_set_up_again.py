@@ -119,3 +119,23 @@ def test_more_k_points_after_the_projectors(num):
     got = ctx.taylor(ctx.upload(many.psi), ctx.zeros(), ctx.zeros(), zc)
     assert S.rel_err(ctx.download(got), O.taylor(many.psi, zc)) < 1e-12
     ctx.close()
+
+
+def test_second_spin_after_v_local():
+    """V_local of one spin, then two spins: H psi is refused until the V_local of
+    both is there; back to one spin, what is there serves on."""
+    from salmon2_b200._lib import SB200Error
+    from salmon2_b200.rt import Context
+    one = _cell((12, 11, 13))
+    psi = synth.random_orbitals(one.grid, np.random.default_rng(6), 2, 2, 1)
+    two = dataclasses.replace(one, nspin=2, rocc=np.full((2, 1, 2), 1.0, order="F"), psi=psi,
+                              V_local=np.asfortranarray(np.concatenate([one.V_local, 1.2 * one.V_local], axis=3)))
+    ctx = Context(one)
+    _set_orbitals(ctx, two)
+    with pytest.raises(SB200Error):
+        ctx.hpsi(ctx.upload(two.psi), ctx.zeros())
+    _set_vlocal(ctx, two.V_local)
+    assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(two.psi), ctx.zeros())), Oracle(two).hpsi(two.psi)) < 1e-12
+    _set_orbitals(ctx, one)
+    assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(one.psi), ctx.zeros())), Oracle(one).hpsi(one.psi)) < 1e-12
+    ctx.close()
