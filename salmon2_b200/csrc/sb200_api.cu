@@ -164,6 +164,12 @@ int upload(T** d, const std::vector<T>& h) {
 // refresh k+A coefficients (and projector phases) for system%vec_Ac
 int refresh_k(sb200_ctx* c) {
   if (!c->g.set || !c->orb.set) return SB200_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  SB_CUDA(cudaStreamIsCapturing(c->stream, &cs));
+  if (cs == cudaStreamCaptureStatusActive) {  // a caller's graph: every replay takes the context's vec_Ac of that time
+    SB_CUDA(cudaMemcpyAsync(c->d_result + 8, c->vec_Ac, 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    return launch_prep_k(c, c->d_result + 8, 0, 0, c->d_kcoef, true);
+  }
   return launch_prep_k(c, nullptr, 4, 0, c->d_kcoef, true);  // vec_Ac by value
 }
 

@@ -1,6 +1,6 @@
 """A context whose grid or orbitals are set again: tables of the earlier shape are
 never used with the new one, and a context set up in steps computes what a
-fresh one does."""
+fresh one does; a vector potential set again between replays of a caller's graph."""
 import ctypes as C
 import dataclasses
 
@@ -138,4 +138,31 @@ def test_second_spin_after_v_local():
     assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(two.psi), ctx.zeros())), Oracle(two).hpsi(two.psi)) < 1e-12
     _set_orbitals(ctx, one)
     assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(one.psi), ctx.zeros())), Oracle(one).hpsi(one.psi)) < 1e-12
+    ctx.close()
+
+
+def test_vector_potential_between_replays():
+    """set_vec_Ac and H psi captured in a graph of the caller's: a replay takes the
+    context's vector potential of that time, not the one of the capture."""
+    import torch
+    from salmon2_b200.rt import Context
+    s = _cell((12, 13, 14))
+    O, ctx, stream = Oracle(s), Context(s), torch.cuda.Stream()
+    ctx.set_stream(stream)
+    psi, out = ctx.upload(s.psi), ctx.zeros()
+    torch.cuda.synchronize()
+    ctx.set_vec_Ac((0.01, 0.0, 0.02))
+    ctx.hpsi(psi, out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        ctx.set_vec_Ac((0.01, 0.0, 0.02))
+        ctx.hpsi(psi, out)
+    for ac in ((-0.03, 0.02, 0.0), (0.0, 0.05, -0.01)):
+        ctx.set_vec_Ac(ac)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        O.set_vec_Ac(ac)
+        assert S.rel_err(ctx.download(out), O.hpsi(s.psi)) < 1e-12
     ctx.close()
