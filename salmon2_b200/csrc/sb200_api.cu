@@ -1353,13 +1353,15 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
   // The first step (nt odd) or two are launched one by one: the device works on
   // them while the rest, two steps (A->B, B->A) at a time, is captured as one
   // CUDA graph, instantiated and replayed.  (With all steps in the graph the
-  // device waited for it, 65 to 75 us a call.)
+  // device waited for it, 65 to 75 us a call.)  A step that the host waits for
+  // outside a graph goes there wherever the count is even.
   cudaGraphExec_t exec2 = nullptr;
   int rc = SB200_OK;
   // with AETRS every step maps A -> A (B its half-step scratch)
   double2* A2 = c->aetrs ? A : B;
   double2* B2 = c->aetrs ? B : A;
-  const int lead = c->timing ? nt : (nt % 2 == 1 ? 1 : std::min(nt, 2));
+  const bool waits = c->gs_interval >= 1 || scf_step_waits(c);
+  const int lead = c->timing ? nt : (nt % 2 == 1 ? 1 : (waits ? 0 : std::min(nt, 2)));
   for (int i = 0; i < lead; ++i) {  // instrumented: every step, its launches bracketed by events
     TRY(i % 2 == 0 ? issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt)
                    : issue_rt_step(c, A2, B2, W, z.data(), n_hamil, trans_longi, dt));

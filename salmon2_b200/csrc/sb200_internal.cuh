@@ -369,6 +369,7 @@ void pcg_default_cells(const sb200_ctx* c, int out[3]);
 int pcg_configure(sb200_ctx* c, int layout, int lmax, const double* rion, int natom, const int npole_xyz[3],
                   double threshold, int maxiter);
 int pcg_issue(sb200_ctx* c, const double* d_rho, double* d_vh, int* iterations);
+bool pcg_host_checked(const sb200_ctx* c);  // the solve's form that the host checks every few iterations
 int pcg_vh_stock(sb200_ctx* c, const int* d_step, int offset, double* d_vh, double* d_s1, double* d_s2, bool before);
 // self-consistent time loop (sb200_scf.cu): buffers sized before a capture, and
 // the per-step potential update issued after each Taylor step (no-ops unless
@@ -385,6 +386,7 @@ int scf_pc_potential(sb200_ctx* c, const double2* psi, const double* vtmp, const
 // stored potentials, the Hartree solve of psi's density, stock update, V_local
 int scf_restart_potential(sb200_ctx* c, const double2* psi);
 bool scf_cg_on(const sb200_ctx* c);
+bool scf_step_waits(const sb200_ctx* c);  // outside a capture the host waits within a self-consistent step
 // the stored potentials of the CG loop (device), or false when there are none
 bool scf_vh_stock(sb200_ctx* c, double** vh, double** s1, double** s2);
 // sum of a device density over the k-point shards (no-op without a communicator)

@@ -1216,10 +1216,11 @@ int pcg_configure(sb200_ctx* c, int layout, int lmax, const double* rion, int na
 }
 
 // One solve of the configured kind: Vh (device, start value in, solution out)
-// of rho (device).  Outside a stream capture the host checks convergence every
-// PCG_CHUNK iterations and *iterations gets poisson%iterVh; inside one the
-// iterations become a conditional WHILE node of the captured graph and
-// *iterations is left alone.
+// of rho (device).  With iterations != null the call waits for the solve and
+// *iterations gets poisson%iterVh.  null (the time loop): the one-launch forms are
+// only launched, a barrier that gave up stays in the context's flag for the end of
+// the loop.  The two-launch form is checked by the host every PCG_CHUNK iterations
+// or, inside a stream capture, becomes a conditional WHILE node of the graph.
 int pcg_issue(sb200_ctx* c, const double* d_rho, double* d_vh, int* iterations) {
   PcgState* s = pcg_of(c);
   if (!s || !s->configured) return set_error(SB200_ERR_STATE, "the CG Hartree solve is not configured");
@@ -1248,14 +1249,14 @@ int pcg_issue(sb200_ctx* c, const double* d_rho, double* d_vh, int* iterations) 
   if (s->solve_grid > 0) {  // every iteration in one cooperative launch
     const cudaError_t le = s->box.g[0] > 0 ? launch_box(a, s->box, st) : launch_solve(a, s->solve_grid, st);
     if (le != cudaSuccess) return cuda_error(le, "CG solve (cooperative launch)");
-    if (cs == cudaStreamCaptureStatusActive) return SB200_OK;
+    if (cs == cudaStreamCaptureStatusActive || !iterations) return SB200_OK;
     SB_CUDA(cudaMemcpyAsync(s->host_sc, a.sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
     SB_CUDA(cudaStreamSynchronize(st));
     if (s->host_sc[SC_DONE] == 3.0) {
       SB_CUDA(cudaMemset(a.err, 0, sizeof(int)));
       return set_error(SB200_ERR_TIMEOUT, "k_pcg_solve: a grid barrier wait expired");
     }
-    if (iterations) *iterations = (int)s->host_sc[SC_ITER];
+    *iterations = (int)s->host_sc[SC_ITER];
     return SB200_OK;
   }
   if (cs == cudaStreamCaptureStatusActive) {
@@ -1297,6 +1298,11 @@ int pcg_issue(sb200_ctx* c, const double* d_rho, double* d_vh, int* iterations) 
   return SB200_OK;
 }
 
+bool pcg_host_checked(const sb200_ctx* c) {
+  const PcgState* s = c->pcg ? static_cast<const PcgState*>(c->pcg) : nullptr;
+  return s != nullptr && s->solve_grid == 0;
+}
+
 int pcg_vh_stock(sb200_ctx* c, const int* d_step, int offset, double* d_vh, double* d_s1, double* d_s2,
                  bool before) {
   const long n = c->g.npts;
@@ -1316,7 +1322,8 @@ int hartree_isolated_cg(sb200_ctx* c, const double* rho, double* vh, int layout,
   if (!rho_dev) SB_CUDA(cudaMemcpyAsync(s->base.rho_stage, rho, n * sizeof(double), cudaMemcpyHostToDevice, st));
   if (!vh_dev) SB_CUDA(cudaMemcpyAsync(s->base.vh_stage, vh, n * sizeof(double), cudaMemcpyHostToDevice, st));
   double* d_vh = vh_dev ? vh : s->base.vh_stage;
-  r = pcg_issue(c, rho_dev ? rho : s->base.rho_stage, d_vh, iterations);
+  int it = 0;
+  r = pcg_issue(c, rho_dev ? rho : s->base.rho_stage, d_vh, iterations ? iterations : &it);
   if (r != SB200_OK) return r;
   if (!vh_dev) {
     SB_CUDA(cudaMemcpyAsync(vh, d_vh, n * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -902,6 +902,11 @@ bool scf_cg_on(const sb200_ctx* c) {
   return s != nullptr && s->cg_on;
 }
 
+bool scf_step_waits(const sb200_ctx* c) {
+  const ScfState* s = c->scf ? static_cast<const ScfState*>(c->scf) : nullptr;
+  return s != nullptr && s->rt_on && s->cg_on && pcg_host_checked(c);
+}
+
 bool scf_vh_stock(sb200_ctx* c, double** vh, double** s1, double** s2) {
   ScfState* s = scf_of(c);
   if (!s || !s->cg_on) return false;
@@ -926,7 +931,8 @@ int scf_restart_potential(sb200_ctx* c, const double2* psi) {
   TRY_S(scf_density_allreduce(c, s->d_rho));
   const double* rho_h = scf_total_density(c, -1);
   TRY_S(pcg_vh_stock(c, s->d_step0, 0, s->d_vh, s->d_stock1, s->d_stock2, true));
-  TRY_S(pcg_issue(c, rho_h, s->d_vh, nullptr));
+  int iterations = 0;
+  TRY_S(pcg_issue(c, rho_h, s->d_vh, &iterations));  // waits: a solve that gave up is an error of this call
   TRY_S(scf_launch_xc(c, s->d_rho, s->d_vxc, -1, false));
   TRY_S(scf_launch_update(c, s->d_vpsl, s->d_vh, s->d_vxc, -1));
   TRY_S(pcg_vh_stock(c, s->d_step0, 0, s->d_vh, s->d_stock1, s->d_stock2, false));
