@@ -1355,27 +1355,27 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
   // CUDA graph, instantiated and replayed.  (With all steps in the graph the
   // device waited for it, 65 to 75 us a call.)  A step that the host waits for
   // outside a graph goes there wherever the count is even.
-  cudaGraphExec_t exec2 = nullptr;
-  int rc = SB200_OK;
   // with AETRS every step maps A -> A (B its half-step scratch)
   double2* A2 = c->aetrs ? A : B;
   double2* B2 = c->aetrs ? B : A;
   const bool waits = c->gs_interval >= 1 || scf_step_waits(c);
   const int lead = c->timing ? nt : (nt % 2 == 1 ? 1 : (waits ? 0 : std::min(nt, 2)));
-  for (int i = 0; i < lead; ++i) {  // instrumented: every step, its launches bracketed by events
-    TRY(i % 2 == 0 ? issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt)
-                   : issue_rt_step(c, A2, B2, W, z.data(), n_hamil, trans_longi, dt));
-    if (c->timing) TRY(timing_flush(c));
-  }
-  const int pairs = (nt - lead) / 2;
-  if (lead % 2 == 1) {  // the graph starts from the odd step's result
-    std::swap(A, A2);
-    std::swap(B, B2);
-  }
-  if (pairs > 0) {
+  auto steps = [&]() -> int {
+    for (int i = 0; i < lead; ++i) {  // instrumented: every step, its launches bracketed by events
+      TRY(i % 2 == 0 ? issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt)
+                     : issue_rt_step(c, A2, B2, W, z.data(), n_hamil, trans_longi, dt));
+      if (c->timing) TRY(timing_flush(c));
+    }
+    const int pairs = (nt - lead) / 2;
+    if (lead % 2 == 1) {  // the graph starts from the odd step's result
+      std::swap(A, A2);
+      std::swap(B, B2);
+    }
+    if (pairs == 0) return SB200_OK;
     cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec2 = nullptr;
     SB_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    rc = issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt);
+    int rc = issue_rt_step(c, A, B, W, z.data(), n_hamil, trans_longi, dt);
     if (rc == SB200_OK) rc = issue_rt_step(c, A2, B2, W, z.data(), n_hamil, trans_longi, dt);
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
     if (rc != SB200_OK) {
@@ -1391,7 +1391,16 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
       if (e != cudaSuccess) rc = cuda_error(e, "cudaGraphLaunch");
     }
     cudaGraphExecDestroy(exec2);
-    if (rc != SB200_OK) return rc;
+    return rc;
+  };
+  const int rc = steps();
+  if (rc != SB200_OK) {  // no step runs on the caller's buffers any more, V_local is the field-free one
+    cudaStreamSynchronize(c->stream);
+    if (c->lg_active) {
+      c->lg_active = 0;
+      if (launch_vloc_restore(c) == SB200_OK) cudaStreamSynchronize(c->stream);
+    }
+    return rc;
   }
   double2* final_buf = nt % 2 == 1 && !c->aetrs ? (double2*)psi_b : (double2*)psi_a;
   if (curr_out && nt > 0)
@@ -1400,14 +1409,13 @@ int sb200_rt_propagate(sb200_ctx* c, double* psi_a, double* psi_b, double* work,
     SB_CUDA(cudaMemcpyAsync(rbox_out, r.d_rbox, 4 * (size_t)nt * sizeof(double), cudaMemcpyDefault, c->stream));
   if (Ac_tot_out)
     SB_CUDA(cudaMemcpyAsync(Ac_tot_out, r.d_Ac_tot, na * sizeof(double), cudaMemcpyDefault, c->stream));
-  SB_CUDA(cudaStreamSynchronize(c->stream));
-  SB_CUDA(cudaGetLastError());
-  TRY(check_device_flag(c));
   if (c->lg_active) {  // the field-free V_local the last step's update_vlocal leaves
     c->lg_active = 0;
     TRY(launch_vloc_restore(c));
-    SB_CUDA(cudaStreamSynchronize(c->stream));
   }
+  SB_CUDA(cudaStreamSynchronize(c->stream));
+  SB_CUDA(cudaGetLastError());
+  TRY(check_device_flag(c));
   r.last_mit = r.loop_mit0 + nt;
   r.last_nt = nt;
   r.start_mit = 0;

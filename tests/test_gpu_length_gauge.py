@@ -85,3 +85,23 @@ def test_length_gauge_is_refused_on_periodic_grids():
     with pytest.raises(_lib.SB200Error):
         ctx.set_length_gauge(True)
     ctx.close()
+
+
+@pytest.mark.parametrize("nt", [4, 5])
+def test_refused_loop_leaves_the_field_free_potential(nt):
+    """A loop whose first step is refused after the field was added to V_local (the
+    mixed form has no absorbing boundary) leaves H psi without the field."""
+    from salmon2_b200 import synth
+    from salmon2_b200._lib import SB200Error
+    from salmon2_b200.rt import Context
+    s = S.isolated_small()
+    ctx, O = Context(s, precision="mixed"), Oracle(s)
+    ctx.set_length_gauge(True)
+    ctx.set_absorbing_boundary(0.3, 2.0)
+    with pytest.raises(SB200Error):
+        ctx.rt_propagate(ctx.upload(s.psi), ctx.zeros(), ctx.zeros(), nt, 0.05, synth.taylor_zc(0.05),
+                         Ac_ext=_pulse(nt, 0.05))
+    ctx.set_precision("fp64")
+    ctx.set_absorbing_boundary(None)
+    assert S.rel_err(ctx.download(ctx.hpsi(ctx.upload(s.psi), ctx.zeros())), O.hpsi(s.psi)) < 1e-12
+    ctx.close()
