@@ -542,14 +542,17 @@ __global__ void __launch_bounds__(1024) k_gram_final(const double* __restrict__ 
 // coefficients of every column follow from G alone.  k_gs_coeff (one CTA)
 // eliminates row after row: row i < j of column j holds T(i, j), the part of
 // the original orbital i in the orthonormal orbital j, rows i >= j what is left
-// of G, so one n x n matrix W (row-major) carries both.  The coefficients
-// carry the rounding of G times the growth |T_ij| |x_i|; when that passes
-// GS_GROWTH (orbitals close to linear dependence, or a zero or non-finite one)
-// *bad is set and the caller takes the column-by-column form instead.  24
+// of G, so one n x n matrix W (row-major) carries both.  Q^T Q = T^T G T carries
+// the rounding of G times the square of the growth g = |T_ij| |x_i|: up to
+// 4 g^2 2^-52 in groups of 5 columns about one other, growth 10 to 70, in 8 to 64
+// of 5814 points; column by column (classical Gram-Schmidt) loses the same square,
+// 1 to 5 times as much there.  When g passes GS_GROWTH (orbitals close to linear
+// dependence, or a zero or non-finite one) *bad is set and the caller takes the
+// column-by-column form instead.  24
 // orbitals of 48^3: 115 launches, 15.7 ms column by column; 5 launches here
 // (a solver iteration with CG and subspace rotation 18.8 -> 2.1 ms).
 // ---------------------------------------------------------------------------
-constexpr double GS_GROWTH = 100.0;  // largest |T_ij| |x_i|: two digits of the 16
+constexpr double GS_GROWTH = 100.0;  // largest |T_ij| |x_i|: its square is four digits of the 16
 constexpr int GC_THREADS = 512;
 constexpr int GC_SMEM_N = 150;  // W kept in shared memory up to here (180 KB)
 

@@ -156,3 +156,32 @@ def test_gram_schmidt_real_all_columns_at_once(no, dependence):
     sl = s.grid.interior_slices()
     X = np.stack([out[sl + (0, i, 0)].ravel() for i in range(no)], axis=1)
     np.testing.assert_allclose(X.T @ X * s.grid.hvol, np.eye(no), atol=4 * no * growth * 2.2e-16)
+
+
+@pytest.mark.parametrize("no,near", [(1, 1.0), (31, 1.0), (33, 1.0), (65, 1.0), (151, 1.0), (8, 0.05), (24, 0.1), (24, 0.015),
+                                     (40, 0.03)], ids=lambda v: str(v))
+def test_gram_schmidt_real_of_a_group_close_together(no, near):
+    """Columns 3 to 7 within `near` of column 2 (growth 1 / near, below the limit at
+    which the column form takes over), and columns far apart at the edges of the
+    tiles.  Against a Householder QR, whose own error is linear in the growth: the
+    coefficients from one Gram matrix lose the growth's square, 4 growth^2 2^-52 in
+    a restatement in numpy; columns far apart keep 1e-14 (here ten times that)."""
+    s = synth.isolated_system(num=(18, 17, 19), no=no, natom=1, seed=60 + no, real=True, name=f"gsnear{no}")
+    rng = np.random.default_rng(no)
+    sl = s.grid.interior_slices()
+    X = rng.standard_normal((18 * 17 * 19, no))
+    X /= np.linalg.norm(X, axis=0)
+    if near < 1.0:
+        X[:, 3:8] = X[:, 2:3] + near * X[:, 3:8]
+    psi0 = np.zeros_like(s.psi)
+    psi0[sl] = X.reshape((18, 17, 19, 1, no, 1), order="F")
+    ctx = _ctx(s)
+    psi = ctx.gs_upload(psi0)
+    ctx.gram_schmidt_real(psi)
+    Q = ctx.gs_download(psi)[sl].reshape(-1, no, order="F") * np.sqrt(s.grid.hvol)
+    ref, r = np.linalg.qr(X)
+    ref *= np.sign(np.diag(r))
+    tol = 1e-13 if near == 1.0 else 16.0 * near ** -2 * 2.2e-16
+    np.testing.assert_allclose(Q.T @ Q, np.eye(no), atol=tol)
+    assert S.rel_err(Q, ref) < tol
+    ctx.close()
