@@ -79,7 +79,7 @@ int ensure_stage(sb200_ctx* c, size_t bytes) {
 
 // (re)allocate work buffers that depend on grid x orbitals x projectors
 int ensure_work(sb200_ctx* c) {
-  c->any_C = -1;  // the shapes of the fused step and the non-orthogonal sweep are chosen anew
+  c->any_C[0] = c->any_C[1] = -1;  // the shapes of the fused step and the non-orthogonal sweep are chosen anew
   c->no_tile = {};
   if (!c->g.set || !c->orb.set) return SB200_OK;
   dfree(c->d_proj);

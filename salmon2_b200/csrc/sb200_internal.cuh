@@ -180,9 +180,10 @@ struct sb200_ctx {
   bool vloc_set = false;
   int vloc_nspin = 0;          // spins d_vloc and d_vloc32 have room for
   NonorthTile no_tile;
-  int any_C = -1;              // cluster size of the fused step of general periodic grids (0: does not apply,
-                               // -1: to be chosen at the next step)
-  int any_resident = 0;        // its clusters at work at a time
+  // the fused step of general periodic grids, of several terms [0] and of one [1]: cluster
+  // size (0: the sweeps; -1: to be chosen at the next step), clusters at work at a time
+  int any_C[2] = {-1, -1};
+  int any_resident[2] = {0, 0};
   int any_smem_cap = 0, any_static = 0;  // dynamic shared memory one of its CTAs can take, its static part
   int stencil_variant = 1;     // 0: per-point reference kernel, 1: tiled 2.5-D sweep
   int orbital_variant = 4;     // 16^3 periodic grids: 4 fused Taylor step with register blocking (when its
@@ -307,6 +308,13 @@ int launch_eigh(sb200_ctx* c, const double* M, int n, double* work, double* V, d
 int launch_hpsi(sb200_ctx* c, const HpsiLaunch& L);
 int launch_hpsi_nonorth(sb200_ctx* c, const HpsiLaunch& L);  // sb200_nonorth.cu
 int launch_hpsi_tiled(sb200_ctx* c, const HpsiLaunch& L);  // sb200_stencil.cu
+// column tiles and z chunks of the two sweeps
+struct SweepShape {
+  int ntiles, zchunk, nzc;
+};
+SweepShape tiled_sweep_shape(const GridInfo& g, int norb);
+SweepShape tma_sweep_shape(const GridInfo& g, int norb, long slots);  // slots: CTAs on the GPU at a time
+bool tma_sweep_applies(const sb200_ctx* c);
 // tensor-copy-fed tiled kernel; SB200_ERR_UNSUPPORTED when it does not apply (sb200_tma_stencil.cu)
 int launch_hpsi_tma(sb200_ctx* c, const HpsiLaunch& L);
 bool orbital_kernel_applies(const sb200_ctx* c);             // sb200_orbital.cu

@@ -684,49 +684,95 @@ void any_limits(sb200_ctx* c) {
   c->any_smem_cap = optin - stat;
 }
 
-// Cluster size for the context's grid, orbitals and projectors (0: the form does
-// not apply), chosen at the first step after one of them was set.
+// Clusters of the shape at work at a time (a cluster stays within a GPC, and GPUs
+// differ in the SMs of theirs: 15 clusters of eight and 33 of four with one CTA per
+// SM on the GPU of the figures below); 0: none.
+int any_resident_clusters(const AnyShape& s, int norb, size_t smem) {
+  cudaLaunchAttribute at;
+  cudaLaunchConfig_t cfg = any_config(s, norb, nullptr, &at);
+  cfg.dynamicSmemBytes = smem;
+  int n = 0;
+  const cudaError_t e = s.stage ? cudaOccupancyMaxActiveClusters(&n, k_step_any<true, true>, &cfg)
+                                : cudaOccupancyMaxActiveClusters(&n, k_step_any<true, false>, &cfg);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+// Microseconds of a time step of four terms with its observables [0], or of one H psi
+// [1], in clusters (any_us) and by the sweeps (sweep_us), from a fit to both over 12
+// grids from 14^3 to 36^3 with 8 and 64 atoms, 1 to 300 orbitals.  In clusters,
+// each wave: the barriers; per column of a thread the planes of the slab and eight of
+// the neighbours', each bound by its own chain of loads (0.7) or by the shared-memory
+// loads of the SM's warps; three passes over the slab's points; the turns of the
+// warps over the atoms.  By the sweeps: waves of two CTAs an SM x planes with their
+// halo, slower once psi and H psi leave L2, and the sphere points of the projections.
+// Rms error 6 and 9 %.  Both sides meet where the last wave is nearly empty or where
+// few large orbitals leave most SMs idle (us, clusters : sweeps, a step): 24^3 32
+// orbitals 113 : 177, 34 orbitals 208 : 177; 36^3 1 orbital 149 : 132, 8 orbitals
+// 148 : 211.  One H psi has a term only to pay for the cluster's prologue: 32^3
+// 8 orbitals 29 : 23; 24^3 300 orbitals 283 : 202; 28^3 300 orbitals 303 : 329.
+double any_us(const sb200_ctx* c, const AnyShape& s, int resident, int alone, int one) {
+  static constexpr double K[2][7] = {{8.5, 0.5, 2.5, 13.6, 4.5, 3.2, 4.1}, {3.2, 2.0, 0.9, 3.4, 0.46, 0.9, 0.4}};
+  const double* k = K[one];
+  const int warps = s.NT / 32, natom = c->pp.nlma > 0 ? c->pp.natom : 0, ncol = c->g.nx * c->g.ny;
+  const int turns = (natom * s.npart + warps - 1) / warps;
+  auto wave = [&](int n) {  // of n clusters; more than `alone` share SMs
+    const double share = n > alone ? 1.0 + 0.4 * ((resident + alone - 1) / alone - 1) : 1.0;
+    const double plane = std::max(0.7, 0.07 * warps * share);
+    return k[0] + (s.C > 1 ? k[1] : 0.0) + s.rounds * plane * (k[2] * s.dmax + k[3]) +
+           share * (k[4] * 1e-3 * s.dmax * ncol + k[s.stage ? 5 : 6] * turns);
+  };
+  const int norb = c->orb.norb, rest = norb % resident;
+  return (one ? 3.5 : 16.5) + (norb / resident) * wave(resident) + (rest > 0 ? wave(rest) : 0.0);
+}
+
+double sweep_us(const sb200_ctx* c, int one) {
+  const int norb = c->orb.norb;
+  const bool tma = tma_sweep_applies(c);
+  const SweepShape s = tma ? tma_sweep_shape(c->g, norb, 296) : tiled_sweep_shape(c->g, norb);
+  const long ctas = (long)s.ntiles * s.nzc * norb, rest = ctas % 296;
+  const double waves = (double)(ctas / 296) + (rest == 0 ? 0.0 : (rest > 148 ? 1.0 : 0.8));
+  const double out = std::min(1.0, std::max(0.0, (32.0 * norb * (double)c->g.npts - 60e6) / 126e6));
+  const double points = 1e-6 * norb * (double)c->pp.totpts;
+  const double h = (c->pp.nlma > 0 ? 0.0 : -3.5) +  // (no launch of projections)
+                   (tma ? 9.0 + waves * (s.zchunk + 8) * (0.9 + 0.35 * out) + 25.0 * points
+                        : 12.0 + waves * (s.zchunk + 8) * (1.1 + 0.5 * out) + 12.0 * points);
+  return one ? h : 5.05 * h;
+}
+
+// Cluster sizes for the context's grid, orbitals and projectors, chosen at the first
+// step after one of them was set.
 void any_plan(sb200_ctx* c) {
-  c->any_C = 0;
+  c->any_C[0] = c->any_C[1] = 0;
   const GridInfo& g = c->g;
   if (!g.set || !c->orb.set || !g.periodic) return;
   if (g.nx == 16 && g.ny == 16 && g.nz == 16) return;  // sb200_orbital_blk.cu
   const PPInfo& pp = c->pp;
   if (pp.nlma > 0 && (pp.npair <= 0 || pp.d_pst == nullptr)) return;  // no (point, atom) pair form
   if ((long)g.nx * g.ny > 4096) return;  // neighbour offsets in 16 bits
+  const char* force = getenv("SB200_CLUSTER");  // this size wherever it fits; 0: the sweeps
   any_limits(c);
   if (c->any_smem_cap == 0) return;
-  const char* force = getenv("SB200_CLUSTER");
-  double best = 0.0;
+  double best[2] = {sweep_us(c, 0), sweep_us(c, 1)};
+  if (force && atoi(force) > 0) best[0] = best[1] = 1e30;
   for (int C = 1; C <= 8; C *= 2) {
     AnyShape s;
     if (force && atoi(force) != C) continue;
     // with the tables in shared memory where they fit
     if (!any_shape(c, C, true, &s) && !any_shape(c, C, false, &s)) continue;
-    // CTAs an SM holds (shared memory, registers, threads), and the clusters at
-    // work at a time: clusters stay within a GPC, which leaves some SMs out
-    // (35 clusters of 4 and 17 of 8 were seen with one CTA per SM)
-    int per_sm = (int)((size_t)(228 * 1024) / (s.smem + c->any_static + 1024));
-    per_sm = std::min(std::min(per_sm, 65536 / (128 * s.NT)), 2048 / s.NT);
-    if (per_sm < 1) continue;
-    const int nclus = (C == 1 ? 148 : 140) * per_sm / C;
-    // cycles of a term, from stamps of the phases on 12^3, 21 x 18 x 15 and 32^3
-    // cells: barriers; the sweep's planes a column, D of its own and eight of the
-    // neighbours', each bound by its own chain of loads (700 cycles) or by the
-    // shared-memory loads of the warps on the SM (70 each), the neighbours' also
-    // by the other CTAs' remote loads; three cycles a point for the rest.  Times
-    // the waves.  (12^3, 32 orbitals: 55, 43, 35 and 43 us with 1, 2, 4 and 8 CTAs;
-    // 21 x 18 x 15, 270 orbitals: 174, 235, 373 and 628.)
-    const double waves = (double)((c->orb.norb + nclus - 1) / nclus);
-    const double share = std::max(1.0, std::min((double)c->orb.norb, (double)nclus) * C / 148.0);  // CTAs per SM
-    const double lds = 70.0 * (s.NT / 32);
-    const double own = std::max(700.0, lds * share), other = (C > 1 ? share : 1.0) * std::max(700.0, lds);
-    const double cost = waves * (3000.0 + (C > 1 ? 2000.0 : 0.0) + s.rounds * (s.dmax * own + 8 * other) +
-                                 3.0 * s.dmax * g.nx * g.ny * share);
-    if (c->any_C == 0 || cost < best) {
-      best = cost;
-      c->any_C = C;
-      c->any_resident = nclus;
+    const int resident = any_resident_clusters(s, c->orb.norb, s.smem);
+    const int alone = any_resident_clusters(s, c->orb.norb, (size_t)c->any_smem_cap);  // one CTA per SM
+    if (resident < 1 || alone < 1) continue;
+    for (int one = 0; one < 2; ++one) {
+      const double us = any_us(c, s, resident, alone, one);
+      if (us < best[one]) {
+        best[one] = us;
+        c->any_C[one] = C;
+        c->any_resident[one] = resident;
+      }
     }
   }
 }
@@ -737,15 +783,16 @@ bool step_any_applies(sb200_ctx* c, int n_hamil) {
   if (c->g.nonorth || c->microac || c->cap_on || c->stencil_variant != 1 || c->sweep_asked ||
       c->project_variant != 1 || c->precision != SB200_PREC_FP64 || n_hamil < 1 || n_hamil > STEP_MAX_NTERM)
     return false;
-  if (c->any_C < 0) any_plan(c);
-  return c->any_C > 0;
+  if (c->any_C[0] < 0) any_plan(c);
+  return c->any_C[n_hamil == 1] > 0;
 }
 
 // hmode: out = H in; else the Taylor step, with_obs: its observables too
 int launch_step_any(sb200_ctx* c, const double2* in, double2* out, const double2* zc, int n_hamil, bool with_obs,
                     bool hmode) {
   AnyShape s;
-  if (!any_shape(c, c->any_C, true, &s) && !any_shape(c, c->any_C, false, &s))
+  const int one = n_hamil == 1, C = c->any_C[one];
+  if (!any_shape(c, C, true, &s) && !any_shape(c, C, false, &s))
     return set_error(SB200_ERR_BAD_SHAPE, "fused step: the orbital does not fit");
   const GridInfo& g = c->g;
   const PPInfo& pp = c->pp;
@@ -803,7 +850,7 @@ int launch_step_any(sb200_ctx* c, const double2* in, double2* out, const double2
   a.o_pm = s.o_pm;
   a.pair_pt = pp.d_pair_pt;
   a.pair_r = pp.d_pair_r;
-  a.ahead = c->any_resident;
+  a.ahead = c->any_resident[one];
   StepZC z;
   for (int i = 0; i < STEP_MAX_NTERM; ++i) z.v[i] = (zc && i < n_hamil) ? zc[i] : make_double2(0.0, 0.0);
   cudaLaunchAttribute at;

@@ -89,28 +89,34 @@ TiledArgs make_tiled_args(const sb200_ctx* c, double2 zc) {
   return a;
 }
 
+// tile: the whole plane for 16x16 periodic grids, else 32x8 (16x16 when the x
+// extent is at most 16); z chunks: enough CTAs to fill the GPU (>= 8 per SM),
+// chunks of >= 8 planes
+SweepShape tiled_sweep_shape(const GridInfo& g, int norb) {
+  SweepShape s;
+  const int TX = g.nx <= 16 ? 16 : 32, TY = TX == 16 ? 16 : 8;
+  s.ntiles = ((g.nx + TX - 1) / TX) * ((g.ny + TY - 1) / TY);
+  const long ctas = (long)s.ntiles * norb;
+  int nchunk = 1;
+  while (ctas * nchunk < 148L * 8 && g.nz / (nchunk * 2) >= 8) nchunk *= 2;
+  s.zchunk = (g.nz + nchunk - 1) / nchunk;
+  s.nzc = (g.nz + s.zchunk - 1) / s.zchunk;
+  return s;
+}
+
 int launch_hpsi_tiled(sb200_ctx* c, const HpsiLaunch& L) {
   const int rt = launch_hpsi_tma(c, L);
   if (rt != SB200_ERR_UNSUPPORTED) return rt;
   TiledArgs a = make_tiled_args(c, L.zc);
-  // tile choice: the whole plane for 16x16 periodic grids, else 32x8 (16x16
-  // when the x extent is at most 16)
   const GridInfo& g = c->g;
   const bool full16 = g.periodic && g.nx == 16 && g.ny == 16;
-  const int TXv = g.nx <= 16 ? 16 : 32;
-  const int TYv = TXv == 16 ? 16 : 8;
-  const int ntiles = ((g.nx + TXv - 1) / TXv) * ((g.ny + TYv - 1) / TYv);
-  // z chunks: enough CTAs to fill the GPU (>= 8 per SM), chunks of >= 8 planes
-  const long ctas = (long)ntiles * c->orb.norb;
-  int nchunk = 1;
-  while (ctas * nchunk < 148L * 8 && g.nz / (nchunk * 2) >= 8) nchunk *= 2;
-  a.zchunk = (g.nz + nchunk - 1) / nchunk;
-  const int nzc = (g.nz + a.zchunk - 1) / a.zchunk;
-  dim3 grid(ntiles, nzc, c->orb.norb);
+  const SweepShape s = tiled_sweep_shape(g, c->orb.norb);
+  a.zchunk = s.zchunk;
+  dim3 grid(s.ntiles, s.nzc, c->orb.norb);
   int r;
   // isolated grids (k + A = 0) skip the gradient terms
   if (full16) r = launch_tiled_t<16, 16, true, true>(L, a, grid, c->stream);
-  else if (TXv == 16) r = g.periodic ? launch_tiled_t<16, 16, false, true>(L, a, grid, c->stream)
+  else if (g.nx <= 16) r = g.periodic ? launch_tiled_t<16, 16, false, true>(L, a, grid, c->stream)
                                      : launch_tiled_t<16, 16, false, false>(L, a, grid, c->stream);
   else r = g.periodic ? launch_tiled_t<32, 8, false, true>(L, a, grid, c->stream)
                       : launch_tiled_t<32, 8, false, false>(L, a, grid, c->stream);

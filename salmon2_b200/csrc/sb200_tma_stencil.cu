@@ -115,14 +115,37 @@ bool make_tma_map(CUtensorMap* m, const void* base, bool f32, const GridInfo& g,
   return r == CUDA_SUCCESS;
 }
 
-// Applies to isolated grids of any shape and to periodic grids with nx = 32
-// and ny a multiple of 8; FP32-input modes need an even nx.  Returns
-// SB200_ERR_UNSUPPORTED (without launching) when the path does not apply.
-int launch_hpsi_tma(sb200_ctx* c, const HpsiLaunch& L) {
+// isolated grids of any shape and periodic grids with nx = 32 and ny a multiple of 8
+bool tma_sweep_applies(const sb200_ctx* c) {
   const GridInfo& g = c->g;
-  if (c->tma_variant == 0) return SB200_ERR_UNSUPPORTED;
+  return c->tma_variant != 0 && (!g.periodic || (g.nx == TX && g.ny % TY == 0 && g.nz >= 1));
+}
+
+// z chunks: the count that minimises waves x planes per CTA (each chunk
+// re-reads 8 halo planes), with the CTAs that fit on the GPU at once
+SweepShape tma_sweep_shape(const GridInfo& g, int norb, long slots) {
+  SweepShape s;
+  s.ntiles = ((g.nx + TX - 1) / TX) * ((g.ny + TY - 1) / TY);
+  const long ctas = (long)s.ntiles * norb;
+  double best = 0.0;
+  for (int n = 1; n <= 16 && (n == 1 || g.nz / n >= 8); ++n) {
+    const int zc = (g.nz + n - 1) / n, nzc = (g.nz + zc - 1) / zc;
+    const double cost = (double)((ctas * nzc + slots - 1) / slots) * (zc + 2 * HALO);
+    if (n == 1 || cost < best) {
+      best = cost;
+      s.zchunk = zc;
+      s.nzc = nzc;
+    }
+  }
+  return s;
+}
+
+// FP32-input modes need an even nx.  Returns SB200_ERR_UNSUPPORTED (without
+// launching) when the path does not apply.
+int launch_hpsi_tma(sb200_ctx* c, const HpsiLaunch& L) {
+  if (!tma_sweep_applies(c)) return SB200_ERR_UNSUPPORTED;
+  const GridInfo& g = c->g;
   const bool per = g.periodic != 0;
-  if (per && !(g.nx == TX && g.ny % TY == 0 && g.nz >= 1)) return SB200_ERR_UNSUPPORTED;
   const bool in32 = L.mode >= 6;
   const int SXv = per ? TX : TX + 2 * HALO;
   const int norb = c->orb.norb;
@@ -135,27 +158,11 @@ int launch_hpsi_tma(sb200_ctx* c, const HpsiLaunch& L) {
   if (acc64 && !make_tma_map(&maps.acc, L.out, false, g, norb, 2 * TX, TY)) return SB200_ERR_UNSUPPORTED;
   if (rd32 && !make_tma_map(&maps.d32, L.d32, true, g, norb, 2 * TX, TY)) return SB200_ERR_UNSUPPORTED;
   TiledArgs a = make_tiled_args(c, L.zc);
-  const int ntiles = ((g.nx + TX - 1) / TX) * ((g.ny + TY - 1) / TY);
-  // z chunks: the count that minimises waves x planes per CTA (each chunk
-  // re-reads 8 halo planes), with the CTAs that fit on the GPU at once
-  const long ctas = (long)ntiles * norb;
   int sms = 148;
   SB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  const long slots = (long)sms * ((L.mode >= 6) ? 3 : 2);
-  int nchunk = 1;
-  double best = 0.0;
-  for (int n = 1; n <= 16 && (n == 1 || g.nz / n >= 8); ++n) {
-    const int zc = (g.nz + n - 1) / n;
-    const int nzc_n = (g.nz + zc - 1) / zc;
-    const double cost = (double)((ctas * nzc_n + slots - 1) / slots) * (zc + 2 * HALO);
-    if (n == 1 || cost < best) {
-      best = cost;
-      nchunk = n;
-    }
-  }
-  a.zchunk = (g.nz + nchunk - 1) / nchunk;
-  const int nzc = (g.nz + a.zchunk - 1) / a.zchunk;
-  dim3 grid(ntiles, nzc, norb);
+  const SweepShape sh = tma_sweep_shape(g, norb, (long)sms * ((L.mode >= 6) ? 3 : 2));
+  a.zchunk = sh.zchunk;
+  dim3 grid(sh.ntiles, sh.nzc, norb);
   return per ? launch_mode<true>(c, maps, L, a, grid) : launch_mode<false>(c, maps, L, a, grid);
 }
 

@@ -1,5 +1,5 @@
 """The cluster-resident fused Taylor step of general periodic grids against the
-oracle: every cluster size, extents that leave partial warps, several columns
+oracle: every cluster size and the sweeps (0), extents that leave partial warps, several columns
 per thread and uneven slabs, one and two spins, with and without projectors;
 H psi alone, one Taylor step, and the time loop's observables."""
 import functools
@@ -38,7 +38,7 @@ CASES = [((12, 12, 12), 1, 2, 2, 8), ((5, 9, 4), 2, 2, 1, 0), ((21, 18, 15), 2, 
          ((32, 32, 16), 1, 1, 1, 6)]
 
 
-@pytest.mark.parametrize("clusters", ["1", "2", "4", "8"])
+@pytest.mark.parametrize("clusters", ["0", "1", "2", "4", "8"])
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(map(str, c[0])))
 def test_cluster_step_against_oracle(case, clusters, monkeypatch):
     from salmon2_b200.rt import Context
@@ -60,3 +60,21 @@ def test_cluster_step_against_oracle(case, clusters, monkeypatch):
     assert S.rel_err(got["curr"], ref["curr"]) < 1e-10
     assert S.rel_err(got["rbox"], ref["rbox"]) < 1e-10
     assert S.rel_err(ctx.download(got["psi"]), ref["psi"]) < 1e-11
+
+
+@pytest.mark.parametrize("no", [1, 32, 34])
+def test_form_chosen_by_the_orbitals_against_oracle(no):
+    """24^3: one wave of clusters (1, 32 orbitals) and one orbital or two more, which
+    the sweeps take; H psi alone chooses for itself."""
+    from salmon2_b200.rt import Context
+    s = _system((24, 24, 24), 1, no, 1, 3)
+    O, ctx = Oracle(s), Context(s)
+    a, b, w = ctx.upload(s.psi), ctx.zeros(), ctx.zeros()
+    assert S.rel_err(ctx.download(ctx.hpsi(a, b)), O.hpsi(s.psi)) < 1e-12
+    nt, zc = 2, synth.taylor_zc(0.04)
+    Ac = synth.asin2cos(nt, 0.04, 0.2, 0.01, 1.0, epdir=(0.3, 0.4, 0.8))
+    ref = O.rt_run(s.psi, nt, 0.04, zc, Ac_ext=Ac)
+    got = ctx.rt_propagate(a, b, w, nt, 0.04, zc, Ac_ext=Ac)
+    assert S.rel_err(got["curr"], ref["curr"]) < 1e-10
+    assert S.rel_err(ctx.download(got["psi"]), ref["psi"]) < 1e-11
+    ctx.close()

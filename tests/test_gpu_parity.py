@@ -372,10 +372,13 @@ def _periodic32():
     return synth.periodic_system(a=10.26, num=16, nkgrid=1, no=2, supercell=2, seed=33, name="periodic32")
 
 
-def test_taylor_parity_periodic32():
-    """Periodic grid with nx = 32: the tensor-copy kernel wraps y and z by
-    coordinates and x inside the tile."""
+@pytest.mark.parametrize("form", ["default", "sweep"])
+def test_taylor_parity_periodic32(form, monkeypatch):
+    """Periodic grid with nx = 32: the default form, and the tensor-copy kernel,
+    which wraps y and z by coordinates and x inside the tile."""
     from salmon2_b200 import synth
+    if form == "sweep":
+        monkeypatch.setenv("SB200_TMA", "on")
     sysm = _periodic32()
     O = Oracle(sysm)
     ctx = _ctx(sysm)
@@ -411,11 +414,15 @@ def test_tensor_copy_kernel_equals_register_sweep(make, precision, monkeypatch):
     assert np.array_equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("form", ["default", "sweep"])
 @pytest.mark.parametrize("trans", ["tr", "lo"])
-def test_rt_propagate_periodic32_current(trans):
-    """32^3 periodic grid: the tensor-copy sweep for H psi and the observables
-    z sweep (shared-memory plane + register window) for J(t) and the dipole."""
+def test_rt_propagate_periodic32_current(trans, form, monkeypatch):
+    """32^3 periodic grid: the default form, and the tensor-copy sweep for H psi with
+    the observables z sweep (shared-memory plane + register window) for J(t) and the
+    dipole."""
     from salmon2_b200 import synth
+    if form == "sweep":
+        monkeypatch.setenv("SB200_TMA", "on")
     sysm = _periodic32()
     nt, dt = 8, 0.08
     Ac = synth.asin2cos(nt, dt, omega=0.05696, f0=0.05696 * 2e-2, tw=nt * dt)
