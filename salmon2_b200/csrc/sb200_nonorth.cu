@@ -19,8 +19,8 @@
 // then done.  The chunk's halo planes take w_x and w_y only.  So psi is read about
 // once and nothing but h and the accumulator is written, where two passes over
 // stored derivatives moved nine blocks (24^3 x 128 orbitals: 120 -> 67 us a term).  Bound by
-// the instructions and shared-memory loads of a point (26 of 16 bytes): the tile
-// is the one that wastes least (tile_shape).
+// the instructions and shared-memory loads of a point (26 of 16 bytes); the tile
+// is the one of the least time by a model of both (tile_shape).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -209,12 +209,17 @@ __global__ void __launch_bounds__(MAX_NT, 2) k_hpsi_no(const double2* __restrict
   }
 }
 
-// The tile and z chunk with the least work per SM: waves x resident warps x
-// planes (8 halo planes each chunk), 0.13 us a warp and plane at any tile.  A
-// thread copies at most SLOTS values of a plane, so narrow tiles get some threads
-// without a column.  24^3 x 128 orbitals: 8 x 8 and whole columns, 16 warps an SM
-// for 32 planes in one wave, 67 us; 24 x 8 tiles, 384 CTAs on 296 places, 98 to
-// 106 us with one to three chunks.
+// The tile and z chunk of the least time: per wave, planes (8 halo planes each chunk)
+// x a chain of 1.3 us, longer with the SM's warps, the values it copies a plane, and
+// the warps whose groups of eight threads straddle rows of the tile (bank conflicts:
+// tiles as wide as the row or a multiple of eight wide are the better ones).  The
+// weights are a fit to 950 pairs of tile and chunk on 11 lattices from 9 x 11 x 30
+// to 40^3, 1 to 200 orbitals; the tile chosen is 0.8 % slower than the best of them
+// on average, 6 % at most.  A thread copies at most SLOTS values of a plane, so
+// narrow tiles get some threads without a column.  H psi, us, the best tile and the
+// one of the least waves x warps x planes with four planes a chunk at least: 26^3 x
+// 2 orbitals 17.5 and 26, x 32 45 and 53; 20^3 x 64 43 and 53; 24^3 x 128 83 both
+// (8 x 8, whole columns).
 NonorthTile tile_shape(const GridInfo& g, int norb) {
   NonorthTile best;
   double least = 0.0;
@@ -231,13 +236,20 @@ NonorthTile tile_shape(const GridInfo& g, int norb) {
       k.NT = (std::max(w * h, (area + SLOTS - 1) / SLOTS) + 31) / 32 * 32;
       k.smem = ((size_t)RING * area + 2 * (size_t)(w + 2 * ND) * h) * sizeof(double2);
       if (k.NT > MAX_NT) continue;
-      const long tiles = (long)((g.nx + w - 1) / w) * ((g.ny + h - 1) / h);
       const int per_sm = std::min(std::min(32, 65536 / (REGS * k.NT)), (int)(SMEM_LIMIT / k.smem));
-      for (k.nchunk = 1; k.nchunk <= 16 && (k.nchunk == 1 || g.nz / k.nchunk >= 4); ++k.nchunk) {
-        const int zc = (g.nz + k.nchunk - 1) / k.nchunk, nzc = (g.nz + zc - 1) / zc;
-        const long ctas = tiles * norb * nzc, slots = 148L * per_sm;
-        const double warps = std::max(8.0, (double)std::min((ctas + 147) / 148, (long)per_sm) * (k.NT / 32));
-        const double cost = (double)((ctas + slots - 1) / slots) * warps * (zc + 2 * ND);
+      const int groups = std::max(1, w * h / 8);
+      int straddle = 0;
+      for (int i = 0; i < groups; ++i) straddle += i * 8 / w != (i * 8 + 7) / w;
+      const double per_cta = 0.006 * (k.NT / 32) + 0.097e-3 * area + 0.012 * ((w * h + 31) / 32) * straddle / groups;
+      const long tiles = (long)((g.nx + w - 1) / w) * ((g.ny + h - 1) / h), slots = 148L * per_sm;
+      for (int nchunk = 1, zc1 = 0; nchunk <= g.nz; ++nchunk) {
+        const int zc = (g.nz + nchunk - 1) / nchunk;
+        if (zc == zc1) continue;
+        zc1 = zc;
+        k.nchunk = nchunk;
+        const long ctas = tiles * norb * ((g.nz + zc - 1) / zc), rest = ctas % slots;
+        const double cost = (zc + 2 * ND) * ((double)(ctas / slots) * (1.3 + per_sm * per_cta) +
+                                             (rest > 0 ? 1.3 + (double)((rest + 147) / 148) * per_cta : 0.0));
         if (best.w == 0 || cost < least) {
           least = cost;
           best = k;

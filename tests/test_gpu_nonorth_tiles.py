@@ -1,7 +1,7 @@
 """The one-sweep non-orthogonal H psi at the edges of its column tiles and z
 chunks, against the oracle: rows of two tiles with a ragged last one, tiles
 wider than a warp, extents of the stencil's reach (the halo wraps onto the tile
-itself), several z chunks, and two spins; H psi and one Taylor step.  1e-12
+itself), z chunks of one plane to all, and two spins; H psi and one Taylor step.  1e-12
 relative, as for the other sizes of this kernel."""
 import numpy as np
 import pytest
@@ -15,7 +15,8 @@ CELL = np.array([[0.60, 0.0, 0.0], [0.16, 0.57, 0.0], [-0.09, 0.19, 0.66]]).T  #
 
 
 @pytest.mark.parametrize("num,no,nspin", [((65, 9, 8), 1, 1), ((9, 41, 11), 2, 1), ((8, 8, 8), 1, 2),
-                                          ((24, 24, 20), 2, 2), ((33, 10, 37), 40, 1)],
+                                          ((24, 24, 20), 2, 2), ((33, 10, 37), 40, 1), ((12, 12, 12), 1, 1),
+                                          ((13, 17, 15), 8, 1), ((20, 20, 20), 34, 1)],
                          ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else str(v))
 def test_tile_edges_against_oracle(num, no, nspin):
     from salmon2_b200 import synth
