@@ -438,6 +438,7 @@ int sb200_ctx_create(int device, sb200_ctx** out) {
     c->tma_variant = (v[0] == 'o' && v[1] == 'f') ? 0 : 1;
     c->sweep_asked = true;
   }
+  if (const char* v = getenv("SB200_CLUSTER")) c->cluster_asked = atoi(v);
   int r = dalloc(&c->d_result, 24);  // results [0, 8), staged A [8, 11), shard sums [16, 23)
   if (r == SB200_OK) r = dalloc(&c->rt.d_step, 1);
   if (r == SB200_OK) r = dalloc(&c->d_err, 1);

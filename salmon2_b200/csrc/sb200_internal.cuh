@@ -198,6 +198,7 @@ struct sb200_ctx {
   int blk_prefetch = 1;        // blocked fused step: each CTA prefetches the orbital one wave ahead into L2
   int tma_variant = 1;         // tiled hpsi fed by tensor copies where it applies (0: register-prefetch sweep)
   bool sweep_asked = false;    // the environment names a sweep: the cluster-resident step stays off
+  int cluster_asked = -1;      // its cluster size in the environment (0: the sweeps, -1: not named)
   // optional per-kernel-class device timing (sb200_set_timing)
   bool timing = false;
   std::vector<cudaEvent_t> ev;  // pairs (start, stop)

@@ -42,7 +42,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <cstdlib>
 #include <type_traits>
 #include <vector>
 
@@ -753,14 +752,15 @@ void any_plan(sb200_ctx* c) {
   const PPInfo& pp = c->pp;
   if (pp.nlma > 0 && (pp.npair <= 0 || pp.d_pst == nullptr)) return;  // no (point, atom) pair form
   if ((long)g.nx * g.ny > 4096) return;  // neighbour offsets in 16 bits
-  const char* force = getenv("SB200_CLUSTER");  // this size wherever it fits; 0: the sweeps
+  const int asked = c->cluster_asked;  // this size wherever it fits; 0: the sweeps
+  if (asked == 0) return;
   any_limits(c);
   if (c->any_smem_cap == 0) return;
   double best[2] = {sweep_us(c, 0), sweep_us(c, 1)};
-  if (force && atoi(force) > 0) best[0] = best[1] = 1e30;
+  if (asked > 0) best[0] = best[1] = 1e30;
   for (int C = 1; C <= 8; C *= 2) {
     AnyShape s;
-    if (force && atoi(force) != C) continue;
+    if (asked > 0 && asked != C) continue;
     // with the tables in shared memory where they fit
     if (!any_shape(c, C, true, &s) && !any_shape(c, C, false, &s)) continue;
     const int resident = any_resident_clusters(s, c->orb.norb, s.smem);
