@@ -75,7 +75,6 @@ struct AnyArgs {
   const int* pt_lin;
   const int* apj;        // [totpts] pair of each sphere point
   const double* uv4;     // [totpts][4]
-  const double* pt_r;    // [totpts][3]
   const double2* phase;  // [nk][totpts]
   const int *lma_start, *nproj;
   const double* rinv;
@@ -824,7 +823,6 @@ int launch_step_any(sb200_ctx* c, const double2* in, double2* out, const double2
   a.ppl = pp.d_ppl;
   a.pt_lin = pp.d_pt_lin;
   a.uv4 = pp.d_uv4;
-  a.pt_r = pp.d_pt_r;
   a.phase = pp.d_phase;
   a.lma_start = pp.d_lma_start;
   a.nproj = pp.d_nproj;

@@ -7,13 +7,15 @@
 // kernels here hold no MMA accumulators in TMEM: they use it as storage that
 // costs neither registers nor shared memory (the Taylor accumulator psi_out,
 // per-point potential and map words), read and written with the 32x32b
-// shape.  Every load / store below waits for its own completion in the same
-// asm statement, so the values are valid as soon as the statement returns.
+// shape.  Every load below, and every store but the _async ones, waits for its
+// own completion in the same asm statement, so the values are valid as soon as
+// the statement returns; after _async stores st_wait() comes before a load.
 //
 // Allocation is by one whole warp; the CTA must hold the columns only while it
-// runs: dealloc them (after a CTA barrier) before the kernel exits.  The
-// kernels that use TMEM run one CTA per SM (their shared memory allows no
-// more), so an allocation never waits for columns held by another CTA.
+// runs: dealloc them (after a CTA barrier) before the kernel exits.  The CTAs of
+// a kernel that share an SM hold a share of its shared memory at least as large
+// as their share of the 512 columns (k_step_blk: one CTA per SM by its registers), so an
+// allocation never waits for columns held by another CTA of the kernel.
 #pragma once
 #include <cuda_runtime.h>
 
