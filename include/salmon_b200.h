@@ -93,7 +93,9 @@ int sb200_kernel_times(sb200_ctx* ctx, double ms[SB200_KIND_COUNT], long count[S
  *                   map of a periodic grid (anything else: SB200_ERR_UNSUPPORTED)
  *   lg_num        : lg%num (global grid size; selects calc_dip's coordinate shift)
  *   hgs           : system%Hgs;  hvol : system%Hvol
- *   coef_lap0, coef_lap(4,3), coef_nab(4,3) : stencil%coef_lap0 / coef_lap / coef_nab */
+ *   coef_lap0, coef_lap(4,3), coef_nab(4,3) : stencil%coef_lap0 / coef_lap / coef_nab
+ * Called again with another extent or periodicity it drops what is given on the
+ * grid: V_local, the projectors, the absorbing boundary, the microscopic field. */
 int sb200_set_grid(sb200_ctx* ctx, const int is[3], const int ie[3], const int is_array[3],
                    const int ie_array[3], const int* idx, const int* idy, const int* idz,
                    const int lg_num[3], const double hgs[3], double hvol, double coef_lap0,
@@ -101,7 +103,8 @@ int sb200_set_grid(sb200_ctx* ctx, const int is[3], const int ie[3], const int i
 
 /* Orbital block: nspin, io = 1..no, ik = 1..nk (info%io_s..io_e, ik_s..ik_e
  * re-based to 1; im = 1), the k-points system%vec_k(3,nk), occupations
- * system%rocc(no,nk,nspin) and weights system%wtk(nk) (src/common/structures.f90:126-203). */
+ * system%rocc(no,nk,nspin) and weights system%wtk(nk) (src/common/structures.f90:126-203).
+ * Called again with a second spin it drops a V_local of one spin. */
 int sb200_set_orbitals(sb200_ctx* ctx, int nspin, int no, int nk, const double* vec_k,
                        const double* rocc, const double* wtk);
 
