@@ -1,7 +1,7 @@
 // sb200_orbital_any.cu -- the fused Taylor step for periodic orthogonal grids
 // of any extents whose orbital fits in the shared memory of a cluster of at
-// most eight CTAs (the default form for them; 16^3 grids have their own,
-// sb200_orbital_blk.cu).
+// most eight CTAs, taken where it is faster than the sweeps (any_us, sweep_us; 16^3
+// grids have their own, sb200_orbital_blk.cu).
 //
 // One thread-block cluster applies all n_hamil terms of taylor.f90:47-117 to
 // one orbital.  CTA r of the C in the cluster holds planes r nz / C ..

@@ -505,12 +505,12 @@ def test_rt_propagate_self_consistent_isolated_cg(nt):
 
 @pytest.mark.parametrize("layout", [1, 3])
 def test_hartree_isolated_cg_one_launch_equals_two_launch_form(layout, monkeypatch):
-    """The CG solve in one cooperative launch (default, grid barriers between
-    the two halves of each iteration) against the two-launch form
-    (SB200_PCG_PERSISTENT=0) on a 64^3 grid, where the one-launch form runs
-    on two blocks per SM: the same iteration count within one and the same
-    potential within 1e-10 relative (the per-block partial sums are cut
-    differently); then a short isolated self-consistent loop with CG under
+    """The CG solve in one cooperative launch, with its vectors on chip (default) and
+    by rows of the grid (SB200_PCG_PERSISTENT=rows, two blocks per SM on this
+    64^3 grid, grid barriers between the two halves of each iteration), against
+    the two-launch form (SB200_PCG_PERSISTENT=0): the same iteration count within
+    one and the same potential within 1e-10 relative (the per-block partial sums
+    are cut differently); then a short isolated self-consistent loop with CG under
     each form: the same orbitals within 1e-10."""
     import dataclasses as dc
     from salmon2_b200 import synth
@@ -520,7 +520,7 @@ def test_hartree_isolated_cg_one_launch_equals_two_launch_form(layout, monkeypat
     s = dc.replace(s0, psi=synth.impulse_kick(s0.grid, s0.psi, 1e-3))
     rho = Oracle(s).density(s.psi)[..., 0]
     out = {}
-    for form in ("1", "0"):
+    for form in ("1", "rows", "0"):
         monkeypatch.setenv("SB200_PCG_PERSISTENT", form)
         ctx = Context(s)
         v, it = ctx.hartree_isolated_cg(rho, layout=layout)
@@ -532,12 +532,14 @@ def test_hartree_isolated_cg_one_launch_equals_two_launch_form(layout, monkeypat
         res = ctx.rt_propagate(a, b, w, 4, 0.05, synth.taylor_zc(0.05))
         out[form] = (v, it, ctx.download(res["psi"]))
         ctx.close()
-    (v1, it1, p1), (v0, it0, p0) = out["1"], out["0"]
-    print(f"CG one launch / two launches, layout {layout}: iterations {it1} / {it0}, "
-          f"potential rel {S.rel_err(v1, v0):.3e}, orbitals rel {S.rel_err(p1, p0):.3e}")
-    assert it1 < 1000 and abs(it1 - it0) <= 1
-    assert S.rel_err(v1, v0) < 1e-10
-    assert S.rel_err(p1, p0) < 1e-10
+    v0, it0, p0 = out["0"]
+    for form in ("1", "rows"):
+        v1, it1, p1 = out[form]
+        print(f"CG one launch ({form}) / two launches, layout {layout}: iterations {it1} / {it0}, "
+              f"potential rel {S.rel_err(v1, v0):.3e}, orbitals rel {S.rel_err(p1, p0):.3e}")
+        assert it1 < 1000 and abs(it1 - it0) <= 1
+        assert S.rel_err(v1, v0) < 1e-10
+        assert S.rel_err(p1, p0) < 1e-10
 
 
 def test_cg_grid_barrier_wait_expires_with_an_error():
