@@ -210,12 +210,12 @@ __global__ void __launch_bounds__(MAX_NT, 2) k_hpsi_no(const double2* __restrict
 }
 
 // The tile and z chunk of the least time: per wave, planes (8 halo planes each chunk)
-// x a chain of 1.3 us, longer with the SM's warps, the values it copies a plane, and
-// the warps whose groups of eight threads straddle rows of the tile (bank conflicts:
-// tiles as wide as the row or a multiple of eight wide are the better ones).  The
-// weights are a fit to 950 pairs of tile and chunk on 11 lattices from 9 x 11 x 30
-// to 40^3, 1 to 200 orbitals; the tile chosen is 0.8 % slower than the best of them
-// on average, 6 % at most.  A thread copies at most SLOTS values of a plane, so
+// x a chain of 1.3 us, longer with the warps behind the CTA's barrier, with the SM's
+// warps, the values it copies a plane, and the warps whose groups of eight threads
+// straddle rows of the tile (bank conflicts: tiles as wide as the row or a multiple
+// of eight wide are the better ones).  The weights are a fit to 2600 pairs of tile
+// and chunk on 13 lattices from 9 x 11 x 30 to 40^3, 1 to 200 orbitals; the tile
+// chosen is 1.3 % slower than the best of them on average, 10 % at most.  A thread copies at most SLOTS values of a plane, so
 // narrow tiles get some threads without a column.  H psi, us, the best tile and the
 // one of the least waves x warps x planes with four planes a chunk at least: 26^3 x
 // 2 orbitals 17.5 and 26, x 32 45 and 53; 20^3 x 64 43 and 53; 24^3 x 128 83 both
@@ -240,7 +240,8 @@ NonorthTile tile_shape(const GridInfo& g, int norb) {
       const int groups = std::max(1, w * h / 8);
       int straddle = 0;
       for (int i = 0; i < groups; ++i) straddle += i * 8 / w != (i * 8 + 7) / w;
-      const double per_cta = 0.006 * (k.NT / 32) + 0.097e-3 * area + 0.012 * ((w * h + 31) / 32) * straddle / groups;
+      const double per_cta = 0.005 * (k.NT / 32) + 0.2e-3 * area + 0.013 * ((w * h + 31) / 32) * straddle / groups;
+      const double chain = 1.3 + 0.014 * (k.NT / 32);
       const long tiles = (long)((g.nx + w - 1) / w) * ((g.ny + h - 1) / h), slots = 148L * per_sm;
       for (int nchunk = 1, zc1 = 0; nchunk <= g.nz; ++nchunk) {
         const int zc = (g.nz + nchunk - 1) / nchunk;
@@ -248,8 +249,8 @@ NonorthTile tile_shape(const GridInfo& g, int norb) {
         zc1 = zc;
         k.nchunk = nchunk;
         const long ctas = tiles * norb * ((g.nz + zc - 1) / zc), rest = ctas % slots;
-        const double cost = (zc + 2 * ND) * ((double)(ctas / slots) * (1.3 + per_sm * per_cta) +
-                                             (rest > 0 ? 1.3 + (double)((rest + 147) / 148) * per_cta : 0.0));
+        const double cost = (zc + 2 * ND) * ((double)(ctas / slots) * (chain + per_sm * per_cta) +
+                                             (rest > 0 ? chain + (double)((rest + 147) / 148) * per_cta : 0.0));
         if (best.w == 0 || cost < least) {
           least = cost;
           best = k;
